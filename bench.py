@@ -152,7 +152,8 @@ class Clocks:
 
 
 # ---------------------------------------------------------------- kernel probe (launch count, per-kernel events)
-KERNELS_PER_CALL = {"b3d_pole_level": 2, "b3d_pole_level_mma": 2, "b3d_cauchy_align": 2, "b3d_cauchy_align_sm": 2}
+KERNELS_PER_CALL = {"b3d_pole_level": 2, "b3d_pole_level_mma": 2, "b3d_cauchy_align": 2, "b3d_cauchy_align_sm": 2,
+                    "b3d_cauchy_align_fp": 2}
 
 
 class Probe:
@@ -499,7 +500,7 @@ def run_ours(args):
     # roofline of the dominant kernel: algorithmic bytes per launch / mean launch time
     L, N, S = op.L, op.plan.Smax ** 2 * (len(ns) if args.schedule == "batched" else 1), op.plan.Smax
     levs = [lv for lv in op.plan.levels if lv]
-    if dominant in ("b3d_cauchy_level", "b3d_cauchy_level2", "b3d_cauchy_level3", "b3d_cauchy_level4"):
+    if dominant in ("b3d_cauchy_level", "b3d_cauchy_level2", "b3d_cauchy_level3", "b3d_cauchy_level4", "b3d_cauchy_level5"):
         per_step_bytes = sum(RL.cauchy_level_bytes(lv, N, L) for lv in levs if lv["m"] > 0 or dominant == "b3d_cauchy_level") \
             * (1 if args.schedule == "batched" else len(ns))
     elif dominant in ("b3d_pole_level", "b3d_pole_level_mma"):

@@ -256,6 +256,34 @@ int b3d_cauchy_level4(int L, const int32_t* xm, const int64_t* xe, int64_t xplan
                                 "b3d_cauchy_level4"));
 }
 
+int b3d_cauchy_fp_size(int L, int64_t dmax, int64_t nb, int64_t Kc, int64_t N, int64_t* doubles) {
+    if (!b3d_supported_limbs(L)) return fail(B3D_E_LIMBS, "no kernels compiled for L = " + std::to_string(L));
+    if (nb < 0 || Kc < 0 || N < 0 || !doubles) return fail(B3D_E_ARG, "b3d_cauchy_fp_size: invalid size");
+    const b3d::CauchyFpTile t = b3d::cauchy_fp_tile(N);
+    *doubles = nb * t.ntile * Kc * b3d::cauchy_fp_digits(L, b3d::cauchy_fp_bits(dmax)) * t.TNp;
+    return 0;
+}
+
+int b3d_cauchy_align_fp(int L, const int32_t* rm, const int64_t* re, int64_t rplane, const b3d_level_tables* lv,
+                        int64_t dmax, double* om, int64_t* oe, void* stream) {
+    if (!level_ok(lv)) return fail(B3D_E_ARG, "b3d_cauchy_align_fp: invalid level description");
+    if (dmax < 1 || dmax >= (1 << 16)) return fail(B3D_E_ARG, "b3d_cauchy_align_fp: dmax must be in [1, 65535]");
+    b3d::CauchyLevel c = level_of(lv);
+    B3D_DISPATCH_CFP(L, cuda_status(FX::align(rm, re, rplane, c, dmax, om, oe, as_stream(stream)), "b3d_cauchy_align_fp"));
+}
+
+int b3d_cauchy_level5(int L, const double* xm, const int64_t* xe, const int32_t* hm, const int64_t* he, int64_t hplane,
+                      const b3d_level_tables* lv, int64_t dmax, int32_t* om, int64_t* oe, int64_t oplane, void* stream) {
+    if (!level_ok(lv)) return fail(B3D_E_ARG, "b3d_cauchy_level5: invalid level description");
+    if (dmax < 1 || dmax >= (1 << 16)) return fail(B3D_E_ARG, "b3d_cauchy_level5: dmax must be in [1, 65535]");
+    if (dmax >= (1 << 10) && lv->Kc >= 2048)
+        return fail(B3D_E_ARG, "b3d_cauchy_level5: more than 2047 columns with divisors from 1024");
+    if (reinterpret_cast<uintptr_t>(xm) % 16) return fail(B3D_E_ARG, "b3d_cauchy_level5: xm not 16-byte aligned");
+    b3d::CauchyLevel c = level_of(lv);
+    B3D_DISPATCH_CFP(L, cuda_status(FX::level(xm, xe, hm, he, hplane, c, dmax, om, oe, oplane, as_stream(stream)),
+                                    "b3d_cauchy_level5"));
+}
+
 int b3d_cauchy_level2(int L, const int32_t* xm, const int64_t* xe, int64_t xplane, const int32_t* hm,
                       const int64_t* he, int64_t hplane, const b3d_level_tables* lv, int32_t* om, int64_t* oe,
                       int64_t oplane, void* stream) {

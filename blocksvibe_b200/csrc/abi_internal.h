@@ -5,9 +5,11 @@
 #include "kernels.cuh"
 #include "rns.cuh"
 #include "cauchy_rns.cuh"
+#include "cauchy_fp.cuh"
 
 namespace b3d {
-#define B3D_DECL(L) extern template struct Launch<L>; extern template struct RnsLaunch<L>; extern template struct CauchyRnsLaunch<L>;
+#define B3D_DECL(L) extern template struct Launch<L>; extern template struct RnsLaunch<L>; extern template struct CauchyRnsLaunch<L>; \
+    extern template struct CauchyFpLaunch<L>;
 B3D_FOR_EACH_L(B3D_DECL)
 #undef B3D_DECL
 
@@ -50,6 +52,22 @@ int cauchy_digits_launch(const CauchyLevel& lv, const uint32_t* table, int64_t d
         case 38: { using CX = b3d::CauchyRnsLaunch<38>; return CALL; }\
         case 46: { using CX = b3d::CauchyRnsLaunch<46>; return CALL; }\
         case 42: { using CX = b3d::CauchyRnsLaunch<42>; return CALL; }         \
+        default: return b3d::fail(B3D_E_LIMBS, "no kernels compiled for L = " + std::to_string(L)); \
+    }
+
+#define B3D_DISPATCH_CFP(L, CALL)                                           \
+    switch (L) {                                                               \
+        case 6: { using FX = b3d::CauchyFpLaunch<6>; return CALL; }           \
+        case 10: { using FX = b3d::CauchyFpLaunch<10>; return CALL; }         \
+        case 18: { using FX = b3d::CauchyFpLaunch<18>; return CALL; }         \
+        case 26: { using FX = b3d::CauchyFpLaunch<26>; return CALL; }         \
+        case 30: { using FX = b3d::CauchyFpLaunch<30>; return CALL; }         \
+        case 34: { using FX = b3d::CauchyFpLaunch<34>; return CALL; }         \
+        case 14: { using FX = b3d::CauchyFpLaunch<14>; return CALL; }\
+        case 22: { using FX = b3d::CauchyFpLaunch<22>; return CALL; }\
+        case 38: { using FX = b3d::CauchyFpLaunch<38>; return CALL; }\
+        case 46: { using FX = b3d::CauchyFpLaunch<46>; return CALL; }\
+        case 42: { using FX = b3d::CauchyFpLaunch<42>; return CALL; }         \
         default: return b3d::fail(B3D_E_LIMBS, "no kernels compiled for L = " + std::to_string(L)); \
     }
 

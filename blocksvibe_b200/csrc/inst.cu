@@ -3,6 +3,7 @@
 #include "kernels.cuh"
 #include "rns.cuh"
 #include "cauchy_rns.cuh"
+#include "cauchy_fp.cuh"
 #include "decimal.cuh"
 #include "pole_mma.cuh"
 
@@ -14,5 +15,6 @@ namespace b3d {
 template struct Launch<B3D_L>;
 template struct RnsLaunch<B3D_L>;
 template struct CauchyRnsLaunch<B3D_L>;
+template struct CauchyFpLaunch<B3D_L>;
 template struct DecimalLaunch<B3D_L>;
 }

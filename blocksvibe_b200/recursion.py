@@ -9,6 +9,7 @@ same bits on the CUDA cores), then the caller's hook (the derivative moments).  
 operator: the M-matrix table, the exact Q values with their sign, q L for every (L, Q) pair of the plan,
 and the R and q L tables aligned per row for the pole step.
 """
+import ctypes
 from fractions import Fraction
 
 import numpy as np
@@ -19,7 +20,7 @@ from .mpf import MPF
 
 
 # default Cauchy kernel and pole-step kernel (see Recursion)
-CAUCHY = "cuda4"
+CAUCHY = "cuda5"
 POLE = "auto"
 # Which pole-step form is faster.  The tensor-core form takes a task's S B columns in chunks of 32 at a cost per
 # chunk that hardly depends on how many columns are in use; the CUDA-core form costs in proportion to the
@@ -41,6 +42,13 @@ def pole_mma_gain(L, S, B):
     return r * cols / (32 * -(-cols // 32))
 
 
+def cauchy_fp_size(L, dmax, nb, Kc, N):
+    """doubles of the digit buffer of b3d_cauchy_align_fp"""
+    n = ctypes.c_int64()
+    _lib.call("b3d_cauchy_fp_size", L, dmax, nb, Kc, N, ctypes.addressof(n))
+    return n.value
+
+
 def _dev(a, device):
     return torch.as_tensor(np.ascontiguousarray(a), dtype=torch.int64).to(device)
 
@@ -53,7 +61,8 @@ class Recursion:
         """cauchy: "cuda" (one-limb divisions on the CUDA cores, b3d_cauchy_level), "cuda2" (the same quotients from
         pre-aligned columns, two per thread, b3d_cauchy_align + b3d_cauchy_level2: bit-identical to "cuda"), "cuda3"
         (cuda2 with 24- or 22-bit quotient digits when the plan's divisors allow, b3d_cauchy_level3: bit-identical), "cuda4"
-        (cuda3 on sign-magnitude columns read limb by limb, b3d_cauchy_align_sm + b3d_cauchy_level4: bit-identical), "rns"
+        (cuda3 on sign-magnitude columns read limb by limb, b3d_cauchy_align_sm + b3d_cauchy_level4: bit-identical), "cuda5"
+        (the quotients by exact double-precision digit steps, b3d_cauchy_align_fp + b3d_cauchy_level5: bit-identical), "rns"
         (the level's Cauchy GEMM on the tensor cores, residues + CRT), or "auto" (rns for levels with at least
         rns_min_k columns, cuda2 below).  pole: "mma" (the pole step's exact sums on the INT8 tensor cores,
         b3d_pole_level_mma; plans with Smax <= 8), "cuda" (b3d_pole_level) or "auto" (mma where the measured
@@ -134,7 +143,7 @@ class Recursion:
         return self._ctable
 
     def _use_rns(self, lev):
-        if self.cauchy in ("cuda", "cuda2", "cuda3", "cuda4") or lev["m"] == 0 or lev["Kc"] > 256:
+        if self.cauchy in ("cuda", "cuda2", "cuda3", "cuda4", "cuda5") or lev["m"] == 0 or lev["Kc"] > 256:
             return False
         return self.cauchy == "rns" or lev["Kc"] >= self.rns_min_k
 
@@ -222,6 +231,14 @@ class Recursion:
                                     p(lev["cold"]), p(lev["ncol"]), p(lev["col"]))
             if self._use_rns(lev):
                 self._cauchy_rns(lev, tabs, res, h_inf, H, stream)
+            elif self.cauchy == "cuda5" and lev["m"] > 0:
+                nb, Kc = lev["nb"], lev["Kc"]
+                Xd = torch.empty(cauchy_fp_size(L, plan.dmax, nb, Kc, N), dtype=torch.float64, device=dev)
+                Xe = torch.empty((nb, N), dtype=torch.int64, device=dev)
+                _lib.call("b3d_cauchy_align_fp", L, p(res.m), p(res.e), res.m.stride(0), _lib.ctypes_byref(tabs),
+                          plan.dmax, p(Xd), p(Xe), stream)
+                _lib.call("b3d_cauchy_level5", L, p(Xd), p(Xe), p(h_inf.m), p(h_inf.e),
+                          h_inf.m.stride(0), _lib.ctypes_byref(tabs), plan.dmax, p(H.m), p(H.e), H.m.stride(0), stream)
             elif self.cauchy == "cuda4" and lev["m"] > 0:
                 nb, Kc = lev["nb"], lev["Kc"]
                 Xm = torch.empty((L, nb * Kc * N), dtype=torch.int32, device=dev)
