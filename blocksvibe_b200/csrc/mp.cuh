@@ -67,15 +67,151 @@ template <int N> B3D_HD void zero(u32 (&a)[N]) {
     for (int k = 0; k < N; k++) a[k] = 0;
 }
 
+// Carry chains.  The carry flag does not survive between asm statements, so a chain runs in statements of eight limbs
+// with the carry in a register between them: 10 instructions per eight limbs against 16 to 32 for carries formed by
+// 64-bit sums or comparisons.
+// r = a + b + c (c <= 1); returns the carry out.  r may be a or b.
+template <int K, int NC, int N> B3D_HD void add_carry_chunk(u32 (&r)[N], const u32 (&a)[N], const u32 (&b)[N], u32& c) {
+#ifdef __CUDA_ARCH__
+    if constexpr (NC == 8) {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "add.cc.u32 t, %8, 0xffffffff;\n\t"
+            "addc.cc.u32 %0, %9, %17;\n\t"
+            "addc.cc.u32 %1, %10, %18;\n\t"
+            "addc.cc.u32 %2, %11, %19;\n\t"
+            "addc.cc.u32 %3, %12, %20;\n\t"
+            "addc.cc.u32 %4, %13, %21;\n\t"
+            "addc.cc.u32 %5, %14, %22;\n\t"
+            "addc.cc.u32 %6, %15, %23;\n\t"
+            "addc.cc.u32 %7, %16, %24;\n\t"
+            "addc.u32 %8, 0, 0;\n\t}"
+            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "=r"(r[K + 4]), "=r"(r[K + 5]), "=r"(r[K + 6]), "=r"(r[K + 7]), "+r"(c)
+            : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(a[K + 4]), "r"(a[K + 5]), "r"(a[K + 6]), "r"(a[K + 7]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]), "r"(b[K + 4]), "r"(b[K + 5]), "r"(b[K + 6]), "r"(b[K + 7]));
+    } else if constexpr (NC == 4) {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "add.cc.u32 t, %4, 0xffffffff;\n\t"
+            "addc.cc.u32 %0, %5, %9;\n\t"
+            "addc.cc.u32 %1, %6, %10;\n\t"
+            "addc.cc.u32 %2, %7, %11;\n\t"
+            "addc.cc.u32 %3, %8, %12;\n\t"
+            "addc.u32 %4, 0, 0;\n\t}"
+            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "+r"(c)
+            : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]));
+    } else if constexpr (NC == 2) {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "add.cc.u32 t, %2, 0xffffffff;\n\t"
+            "addc.cc.u32 %0, %3, %5;\n\t"
+            "addc.cc.u32 %1, %4, %6;\n\t"
+            "addc.u32 %2, 0, 0;\n\t}"
+            : "=r"(r[K + 0]), "=r"(r[K + 1]), "+r"(c)
+            : "r"(a[K + 0]), "r"(a[K + 1]), "r"(b[K + 0]), "r"(b[K + 1]));
+    } else {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "add.cc.u32 t, %1, 0xffffffff;\n\t"
+            "addc.cc.u32 %0, %2, %3;\n\t"
+            "addc.u32 %1, 0, 0;\n\t}"
+            : "=r"(r[K + 0]), "+r"(c)
+            : "r"(a[K + 0]), "r"(b[K + 0]));
+    }
+#else
+    for (int k = K; k < K + NC; k++) {
+        const u64 v = (u64)a[k] + b[k] + c;
+        r[k] = (u32)v;
+        c = (u32)(v >> 32) & 1u;
+    }
+#endif
+}
+
+template <int K, int N> B3D_HD void add_carry_from(u32 (&r)[N], const u32 (&a)[N], const u32 (&b)[N], u32& c) {
+    if constexpr (K < N) {
+        constexpr int NC = N - K >= 8 ? 8 : (N - K >= 4 ? 4 : (N - K >= 2 ? 2 : 1));
+        add_carry_chunk<K, NC, N>(r, a, b, c);
+        add_carry_from<K + NC, N>(r, a, b, c);
+    }
+}
+
+template <int N> B3D_HD u32 add_carry(u32 (&r)[N], const u32 (&a)[N], const u32 (&b)[N], u32 c) {
+    add_carry_from<0, N>(r, a, b, c);
+    return c;
+}
+
+// r = a - b - c (c <= 1); returns the borrow out.  r may be a or b.
+template <int K, int NC, int N> B3D_HD void sub_borrow_chunk(u32 (&r)[N], const u32 (&a)[N], const u32 (&b)[N], u32& c) {
+#ifdef __CUDA_ARCH__
+    if constexpr (NC == 8) {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "sub.cc.u32 t, 0, %8;\n\t"
+            "subc.cc.u32 %0, %9, %17;\n\t"
+            "subc.cc.u32 %1, %10, %18;\n\t"
+            "subc.cc.u32 %2, %11, %19;\n\t"
+            "subc.cc.u32 %3, %12, %20;\n\t"
+            "subc.cc.u32 %4, %13, %21;\n\t"
+            "subc.cc.u32 %5, %14, %22;\n\t"
+            "subc.cc.u32 %6, %15, %23;\n\t"
+            "subc.cc.u32 %7, %16, %24;\n\t"
+            "subc.u32 %8, 0, 0;\n\tand.b32 %8, %8, 1;\n\t}"
+            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "=r"(r[K + 4]), "=r"(r[K + 5]), "=r"(r[K + 6]), "=r"(r[K + 7]), "+r"(c)
+            : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(a[K + 4]), "r"(a[K + 5]), "r"(a[K + 6]), "r"(a[K + 7]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]), "r"(b[K + 4]), "r"(b[K + 5]), "r"(b[K + 6]), "r"(b[K + 7]));
+    } else if constexpr (NC == 4) {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "sub.cc.u32 t, 0, %4;\n\t"
+            "subc.cc.u32 %0, %5, %9;\n\t"
+            "subc.cc.u32 %1, %6, %10;\n\t"
+            "subc.cc.u32 %2, %7, %11;\n\t"
+            "subc.cc.u32 %3, %8, %12;\n\t"
+            "subc.u32 %4, 0, 0;\n\tand.b32 %4, %4, 1;\n\t}"
+            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "+r"(c)
+            : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]));
+    } else if constexpr (NC == 2) {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "sub.cc.u32 t, 0, %2;\n\t"
+            "subc.cc.u32 %0, %3, %5;\n\t"
+            "subc.cc.u32 %1, %4, %6;\n\t"
+            "subc.u32 %2, 0, 0;\n\tand.b32 %2, %2, 1;\n\t}"
+            : "=r"(r[K + 0]), "=r"(r[K + 1]), "+r"(c)
+            : "r"(a[K + 0]), "r"(a[K + 1]), "r"(b[K + 0]), "r"(b[K + 1]));
+    } else {
+        asm("{\n\t.reg .u32 t;\n\t"
+            "sub.cc.u32 t, 0, %1;\n\t"
+            "subc.cc.u32 %0, %2, %3;\n\t"
+            "subc.u32 %1, 0, 0;\n\tand.b32 %1, %1, 1;\n\t}"
+            : "=r"(r[K + 0]), "+r"(c)
+            : "r"(a[K + 0]), "r"(b[K + 0]));
+    }
+#else
+    for (int k = K; k < K + NC; k++) {
+        const u64 v = (u64)a[k] - b[k] - c;
+        r[k] = (u32)v;
+        c = (u32)(v >> 32) & 1u;
+    }
+#endif
+}
+
+template <int K, int N> B3D_HD void sub_borrow_from(u32 (&r)[N], const u32 (&a)[N], const u32 (&b)[N], u32& c) {
+    if constexpr (K < N) {
+        constexpr int NC = N - K >= 8 ? 8 : (N - K >= 4 ? 4 : (N - K >= 2 ? 2 : 1));
+        sub_borrow_chunk<K, NC, N>(r, a, b, c);
+        sub_borrow_from<K + NC, N>(r, a, b, c);
+    }
+}
+
+template <int N> B3D_HD u32 sub_borrow(u32 (&r)[N], const u32 (&a)[N], const u32 (&b)[N], u32 c) {
+    sub_borrow_from<0, N>(r, a, b, c);
+    return c;
+}
+
+// r = a + c (c <= 1)
+template <int N> B3D_HD u32 add_bit(u32 (&r)[N], const u32 (&a)[N], u32 c) {
+    u32 z[N];
+    zero(z);
+    return add_carry(r, a, z, c);
+}
+
 // two's complement negation in place
 template <int N> B3D_HD void negate(u32 (&a)[N]) {
-    u32 c = 1;
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        u32 v = ~a[k] + c;
-        c = (c && v == 0) ? 1u : 0u;
-        a[k] = v;
-    }
+    u32 z[N];
+    zero(z);
+    sub_borrow(a, z, a, 0u);
 }
 
 template <int N> B3D_HD bool is_zero(const u32 (&a)[N]) {
@@ -184,14 +320,10 @@ template <int L, int NW> B3D_HD bool round_mag(const u32 (&w)[NW], i64 ein, u32 
     }
     u32 t[L + 1];
     shr(w, s - 1, t);                      // keeps the rounding bit in bit 0
-    u32 c = t[0] & 1u;
+    const u32 half = t[0] & 1u;
 #pragma unroll
-    for (int k = 0; k < L; k++) {
-        u32 v = (t[k] >> 1) | (t[k + 1] << 31);
-        u32 sum = v + c;
-        c = (c && sum == 0) ? 1u : 0u;
-        r[k] = sum;
-    }
+    for (int k = 0; k < L; k++) r[k] = fsr(t[k], t[k + 1], 1);
+    add_bit(r, r, half);
     // a carry out of bit NB - 1 makes the magnitude 2^NB: renormalise
     if ((r[L - 1] >> (NB - 32 * (L - 1))) != 0) {
         u32 q[L];
@@ -368,26 +500,13 @@ template <int L> B3D_HD void add_norm(const u32 (&a)[L], bool na, i64 ea, const 
     if (ds >= 0) shl(sm, (int)ds, t); else shr(sm, (int)(-ds > 64 * L ? 64 * L : -ds), t);
     // magnitudes: |big| 2^32 +- |small|, one carry (or borrow) chain; a borrow out means |small| was larger
     bool neg = sbig;
+#pragma unroll
+    for (int k = 1; k <= L; k++) acc[k] = abig ? a[k - 1] : b[k - 1];
     if (sbig == ssmall) {
-        u32 c = 0;
-#pragma unroll
-        for (int k = 0; k < L + 2; k++) {
-            const u64 v = (u64)(k >= 1 && k <= L ? (abig ? a[k - 1] : b[k - 1]) : 0u) + t[k] + c;
-            acc[k] = (u32)v;
-            c = (u32)(v >> 32);
-        }
-    } else {
-        u32 br = 0;
-#pragma unroll
-        for (int k = 0; k < L + 2; k++) {
-            const u64 v = (u64)(k >= 1 && k <= L ? (abig ? a[k - 1] : b[k - 1]) : 0u) - t[k] - br;
-            acc[k] = (u32)v;
-            br = (u32)(v >> 63);
-        }
-        if (br) {
-            negate(acc);
-            neg = !neg;
-        }
+        add_carry(acc, acc, t, 0u);
+    } else if (sub_borrow(acc, acc, t, 0u)) {
+        negate(acc);
+        neg = !neg;
     }
     if (!round_mag<L>(acc, T, r, er)) { *nr = false; return; }
     *nr = neg;
@@ -443,29 +562,15 @@ template <int L> B3D_HD void add_norm_col(const u32 (&a)[L], bool na, i64 ea, co
         lo = hi;
     }
     u32 acc[L + 2];
+    zero(acc);
     bool neg = sbig;
+#pragma unroll
+    for (int k = 1; k <= L; k++) acc[k] = abig ? a[k - 1] : b[(k - 1) * stride];
     if (sbig == ssmall) {
-        u32 c = 0;
-#pragma unroll
-        for (int k = 0; k < L + 2; k++) {
-            const u32 big = (k >= 1 && k <= L) ? (abig ? a[k - 1] : b[(k - 1) * stride]) : 0u;
-            const u64 v = (u64)big + t[k] + c;
-            acc[k] = (u32)v;
-            c = (u32)(v >> 32);
-        }
-    } else {
-        u32 br = 0;
-#pragma unroll
-        for (int k = 0; k < L + 2; k++) {
-            const u32 big = (k >= 1 && k <= L) ? (abig ? a[k - 1] : b[(k - 1) * stride]) : 0u;
-            const u64 v = (u64)big - t[k] - br;
-            acc[k] = (u32)v;
-            br = (u32)(v >> 63);
-        }
-        if (br) {
-            negate(acc);
-            neg = !neg;
-        }
+        add_carry(acc, acc, t, 0u);
+    } else if (sub_borrow(acc, acc, t, 0u)) {
+        negate(acc);
+        neg = !neg;
     }
     if (!round_mag<L>(acc, T, r, er)) { *nr = false; return; }
     *nr = neg;
