@@ -75,6 +75,25 @@ __device__ __forceinline__ uint32_t barrett(uint64_t x, uint32_t p, uint64_t mu)
     return (uint32_t)r;
 }
 
+// x mod p for p = 2^31 - c with c < kNearC: two folds x = (x mod 2^31) + c (x / 2^31) and one conditional subtraction
+// (x < 2^62: the first fold leaves less than 2^31 + 2^44, the second less than 2^31 + 2^27).  9 instructions against
+// some 20 of the Barrett step.
+constexpr uint32_t kNearC = 8192;
+__device__ __forceinline__ uint32_t mod_near(uint64_t x, uint32_t p, uint32_t c) {
+    const uint64_t y = (uint64_t)(uint32_t)(x >> 31) * c + ((uint32_t)x & 0x7FFFFFFFu);
+    const uint32_t r = (uint32_t)(y >> 31) * c + ((uint32_t)y & 0x7FFFFFFFu);
+    return min(r, r - p);
+}
+
+// hi 2^16 + lo
+__device__ __forceinline__ uint64_t widen16(uint32_t hi, uint32_t lo) { return (uint64_t)hi * 65536u + lo; }
+
+// the same for x < 1.1 2^48: one fold (below 2^31 + 1.1 2^30)
+__device__ __forceinline__ uint32_t mod_near48(uint64_t x, uint32_t p, uint32_t c) {
+    const uint32_t r = (uint32_t)(x >> 31) * c + ((uint32_t)x & 0x7FFFFFFFu);
+    return min(r, r - p);
+}
+
 // ------------------------------------------------------------------------------------------------
 // 1. digits.  Element (b, r, k) of a strided aligned operand (two's complement limb planes, plane stride
 // `plane`, element index b * sb + r * sr + k * sk) -> digits of its residues at rows 4 r + s, column k of the
@@ -418,7 +437,8 @@ __global__ void __launch_bounds__(256, 2) k_rns_mma4(RnsMma a, RnsTables tb) {
 
         const uint32_t p = __ldg(tb.p + j);
         const uint64_t mu = __ldg(tb.mu + j);
-        const uint32_t inv = __ldg(tb.inv + j);
+        const uint32_t inv = __ldg(tb.inv + j), pc = 0x80000000u - p;
+        const bool near = pc < kNearC;
         uint32_t w[7];
 #pragma unroll
         for (int u = 0; u < 7; u++) w[u] = __ldg(tb.w + j * 8 + u);
@@ -432,24 +452,46 @@ __global__ void __launch_bounds__(256, 2) k_rns_mma4(RnsMma a, RnsTables tb) {
                   "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
                 : "r"(taddr + (uint32_t)c0));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            // partial sums of the four outputs q of this chunk (this lane's row digit s), then a
-            // reduce-scatter over the four lanes of the row: lane s ends with the full sum of output q = s
-            uint64_t pq[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                uint64_t v = 0;
-#pragma unroll
-                for (int t = 0; t < 4; t++) v += (uint64_t)d[4 * q + t] * w[s + t];
-                pq[q] = v;
-            }
             const bool hi2 = (s & 2) != 0, hi1 = (s & 1) != 0;
-            const uint64_t k0 = hi2 ? pq[2] : pq[0], k1 = hi2 ? pq[3] : pq[1];
-            const uint64_t x0 = hi2 ? pq[0] : pq[2], x1 = hi2 ? pq[1] : pq[3];
-            const uint64_t a0 = k0 + __shfl_xor_sync(0xFFFFFFFFu, x0, 2);     // outputs (s & 2) + {0, 1}
-            const uint64_t a1 = k1 + __shfl_xor_sync(0xFFFFFFFFu, x1, 2);
-            const uint64_t v = (hi1 ? a1 : a0) + __shfl_xor_sync(0xFFFFFFFFu, hi1 ? a0 : a1, 1);   // output s
-            const uint32_t r = barrett(v, p, mu);
-            const uint32_t y = barrett((uint64_t)r * inv, p, mu);
+            uint32_t y;
+            if (near) {
+                // the four outputs' column digits folded and reduced per lane (row digit s), the four lanes of a row
+                // exchanged (lane s ends with the four row digits of output s), folded and reduced again; 32-bit
+                // exchanges and cheap reductions: 66 instructions per 16 sums against some 110 of the general form
+                uint32_t f[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    f[q] = mod_near48((uint64_t)d[4 * q] + (uint64_t)d[4 * q + 1] * 256u + (uint64_t)d[4 * q + 2] * 65536u +
+                                      (uint64_t)d[4 * q + 3] * 16777216u, p, pc);
+                const uint32_t k0 = hi2 ? f[2] : f[0], k1 = hi2 ? f[3] : f[1];          // kept: outputs (s & 2) + {0, 1}
+                const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, hi2 ? f[0] : f[2], 2);  // the same from row digit s ^ 2
+                const uint32_t g1 = __shfl_xor_sync(0xFFFFFFFFu, hi2 ? f[1] : f[3], 2);
+                const uint32_t u0 = hi1 ? k1 : k0, u2 = hi1 ? g1 : g0;                   // output s: digits s and s ^ 2
+                const uint32_t u1 = __shfl_xor_sync(0xFFFFFFFFu, hi1 ? k0 : k1, 1);      // digits s ^ 1 and s ^ 3
+                const uint32_t u3 = __shfl_xor_sync(0xFFFFFFFFu, hi1 ? g0 : g1, 1);
+                const uint32_t a0 = hi1 ? u1 : u0, a1 = hi1 ? u0 : u1, a2 = hi1 ? u3 : u2, a3 = hi1 ? u2 : u3;
+                const uint64_t lo = (uint64_t)a1 * 256u + a0, hi = (uint64_t)a3 * 256u + a2;
+                const uint32_t r = mod_near((hi2 ? hi : lo) + (hi2 ? lo : hi) * 65536u, p, pc);   // < 2^56
+                y = mod_near((uint64_t)r * inv, p, pc);
+            } else {
+                // partial sums of the four outputs q of this chunk (this lane's row digit s), then a
+                // reduce-scatter over the four lanes of the row: lane s ends with the full sum of output q = s
+                uint64_t pq[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    uint64_t v = 0;
+#pragma unroll
+                    for (int t = 0; t < 4; t++) v += (uint64_t)d[4 * q + t] * w[s + t];
+                    pq[q] = v;
+                }
+                const uint64_t k0 = hi2 ? pq[2] : pq[0], k1 = hi2 ? pq[3] : pq[1];
+                const uint64_t x0 = hi2 ? pq[0] : pq[2], x1 = hi2 ? pq[1] : pq[3];
+                const uint64_t a0 = k0 + __shfl_xor_sync(0xFFFFFFFFu, x0, 2);     // outputs (s & 2) + {0, 1}
+                const uint64_t a1 = k1 + __shfl_xor_sync(0xFFFFFFFFu, x1, 2);
+                const uint64_t v = (hi1 ? a1 : a0) + __shfl_xor_sync(0xFFFFFFFFu, hi1 ? a0 : a1, 1);   // output s
+                const uint32_t r = barrett(v, p, mu);
+                y = barrett((uint64_t)r * inv, p, mu);
+            }
             const int ll = c0 / 4 + s;
             *reinterpret_cast<uint32_t*>(ysm + ((size_t)(row >> 2) * (TN / 4) + ll) * 16 + 4 * pi) = y;
         }
@@ -484,12 +526,20 @@ __global__ void __launch_bounds__(256, 2) k_rns_mma4(RnsMma a, RnsTables tb) {
 #endif
 
 // ------------------------------------------------------------------------------------------------
-// 1'. digits on the tensor cores.  One CTA = a tile of 8 operand rows x 16 columns k (128 elements).  The
-// elements' magnitude bytes form A (128 rows x 4 L bytes, K-major in shared memory); the constant
-// C[(j, t)][d] = byte t of (2^(8 d) mod p_j) is B (two tiles of NS rows); S = A B^T holds
-// sum_d digit_d C[(j, t)][d] < 4 L 255^2, so r_j = sum_t S[4 j + t] 2^(8 t) mod p_j (sign applied after).
-// The residue digits are staged in shared memory and written as 16-byte chunks of the same K-major
-// digit matrices k_rns_split writes.
+// 1'. digits on the tensor cores.  One tile = 8 operand rows x 16 columns k (128 elements).  The elements' bytes of the
+// magnitude) form A (128 rows x 4 L bytes, K-major in shared memory); the constant C[(j, t)][d] = byte t of
+// (2^(8 d) mod p_j) is B (two tiles of NS rows); S = A B^T holds sum_d byte_d C[(j, t)][d] < 4 L 255^2, so
+// r_j = sum_t S[4 j + t] 2^(8 t) mod p_j (sign applied after).
+//
+// A CTA (256 threads, two per SM) is persistent over the tiles: each tile's MMAs go out in four chunks of at most
+// 128 columns on two TMEM buffers, so that the reduction of one chunk runs while the next is multiplied, and the
+// next tile's limbs are on their way into registers.  The reduction is what bounds it: about 20 instructions per
+// residue.  The primes lie just below 2^31, so with c = 2^31 - p one step v = (v mod 2^31) + c (v / 2^31) and one
+// conditional subtraction reduce (a prime with a larger c takes the Barrett step).  The four digit bytes of four
+// neighbouring k are transposed by two shuffles, so that a warp stores 128 contiguous bytes of the digit matrix per
+// prime, straight from registers: with byte stores to a shared-memory stage, one warp per 32 elements and (1472 bits)
+// one CTA of four warps per SM, the form before took 50.3 ms per 1280-bit task and 8.7 per 1024-bit task, 19.5 and 3.7
+// here.
 struct RnsSplit {
     const int32_t* m; int64_t plane, nb, R, K, sb, sr, sk;   // aligned operand
     int64_t Rp, Kp; int TR; int64_t mat_bytes;               // output digit matrices
@@ -500,33 +550,44 @@ struct RnsSplit {
 };
 
 #ifdef B3D_DEFINE_LAUNCH
+B3D_CX int rns_split_smem(int Ks, int NS, int np) { return 128 * Ks + 2 * NS * Ks + (np + 3) / 4 * 32; }
+
+// In the reduction the four lanes of four neighbouring k exchange bytes in two steps, so that lane q of the four ends
+// with byte q of each lane's residue (sel1, sel2: the lane's byte selectors).
 template <int L>
-__global__ void __launch_bounds__(128, 1) k_rns_split_mma(RnsSplit a, RnsTables tb) {
+__global__ void __launch_bounds__(256, 2) k_rns_split_mma(RnsSplit a, RnsTables tb) {
+    constexpr int LH = (L / 2 + 3) / 4 * 4;              // limbs loaded by the first of an element's two threads
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bar_load, bar_mma;
+    __shared__ __align__(8) uint64_t bar_load, bar_mma[2];
     __shared__ uint32_t tmem_base_sh;
     __shared__ int fail_sh;
     __shared__ uint8_t neg_sh[128];
     const int Ks = a.Ks, NS = a.NS, np = tb.np;
-    uint8_t* sA = smem;                                  // 128 x Ks magnitude bytes
+    uint8_t* sA = smem;                                  // 128 x Ks operand bytes
     uint8_t* sC = smem + 128 * Ks;                       // 2 NS x Ks constants
-    uint8_t* sD = sC + 2 * NS * Ks;                      // np x 4 x 8 x 16 staged digits
-    const int warp = threadIdx.x / 32, t = threadIdx.x;
+    uint2* tab = reinterpret_cast<uint2*>(sC + 2 * NS * Ks);   // p, 2^31 - p
+    const int t = threadIdx.x, warp = t / 32, lane = t % 32;
     const int64_t ktiles = a.Kp / 16, tiles = ktiles * ((a.Rp + 7) / 8), items = tiles * a.nb;
-    const uint32_t ncols = 256;                          // one half (NS <= 256 columns) at a time
     if (t == 0) {
         fail_sh = 0;
         mbar_init(&bar_load, 1);
-        mbar_init(&bar_mma, 1);
+        mbar_init(&bar_mma[0], 1);
+        mbar_init(&bar_mma[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_base_sh)), "r"(ncols) : "memory");
+                     ::"r"(smem_u32(&tmem_base_sh)), "r"(256) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    int far = 0;
+    for (int j = t; j < (np + 3) / 4 * 4; j += blockDim.x) {
+        const uint32_t p = __ldg(tb.p + (j < np ? j : 0));
+        tab[j] = make_uint2(p, 0x80000000u - p);
+        far |= 0x80000000u - p >= kNearC;
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    const bool near = !__syncthreads_or(far);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_sh;
     if (t == 0) {
@@ -537,114 +598,157 @@ __global__ void __launch_bounds__(128, 1) k_rns_split_mma(RnsSplit a, RnsTables 
     if (!mbar_wait(&bar_load, 0, kWaitLimit)) atomicExch(&fail_sh, 1);
     __syncthreads();
     bool run = fail_sh == 0;
-    int mma_h = 0;                                        // pass of the last MMA commit (failure drain)
-    // persistent: the constant and the TMEM allocation serve every tile this CTA takes
-    for (int64_t item = blockIdx.x; item < items && run; item += gridDim.x) {
-    const int64_t b = item / tiles, tile = item % tiles;
-    const int64_t r0 = (tile / ktiles) * 8, k0 = (tile % ktiles) * 16;
-    // magnitudes of the tile's elements -> A rows e = rr * 16 + kk (load order follows the unit stride)
-    {
-        const bool rows_fast = a.sr == 1;
-        const int rr = rows_fast ? (t % 8) : (t / 16), kk = rows_fast ? (t / 8) : (t % 16);
-        const int e = rr * 16 + kk;
-        const int64_t r = r0 + rr, k = k0 + kk;
-        u32 v[L];
-        bool neg = false;
-        if (r < a.R && k < a.K) neg = load_mag<L>(a.m, a.plane, b * a.sb + r * a.sr + k * a.sk, v);
-        else zero(v);
-        neg_sh[e] = neg;
+
+    // loading: two threads per element (limbs [0, LH) and [LH, L)); eight k x four rows per warp where the rows are
+    // contiguous (sr = 1), 16 k x 2 rows otherwise; element e = rr 16 + kk either way
+    const bool rows_fast = a.sr == 1;
+    const int half = t >> 7, t7 = t & 127;
+    const int lr = rows_fast ? (t7 >> 3) & 7 : t7 >> 4, lk = rows_fast ? (t7 & 7) + 8 * (t7 >> 6) : t7 & 15, le = lr * 16 + lk;
+    // magnitude bytes without a carry between the two threads: a negative element is stored complemented and the
+    // missing one is added to its residues' sums
+    u32 v[LH];
+    bool vneg = false;
+    auto load = [&](int64_t item) {
+        const int64_t b = item / tiles, tile = item % tiles;
+        const int64_t r = (tile / ktiles) * 8 + lr, k = (tile % ktiles) * 16 + lk;
+        const bool ok = r < a.R && k < a.K;
+        const int32_t* src = a.m + b * a.sb + r * a.sr + k * a.sk + (half ? LH * a.plane : 0);
 #pragma unroll
-        for (int c = 0; c < (4 * L + 15) / 16; c++) {
-            uint4 w;
-            w.x = 4 * c + 0 < L ? v[4 * c + 0] : 0u;
-            w.y = 4 * c + 1 < L ? v[4 * c + 1] : 0u;
-            w.z = 4 * c + 2 < L ? v[4 * c + 2] : 0u;
-            w.w = 4 * c + 3 < L ? v[4 * c + 3] : 0u;
-            *reinterpret_cast<uint4*>(sA + tiled_offset(e, 16 * c, 128, Ks)) = w;
-        }
-        for (int c = (4 * L + 15) / 16; c < Ks / 16; c++)
-            *reinterpret_cast<uint4*>(sA + tiled_offset(e, 16 * c, 128, Ks)) = make_uint4(0, 0, 0, 0);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // generic-proxy writes -> tensor core
-    __syncthreads();
-    // two passes over the halves of the constant matrix, sharing 256 TMEM columns (two CTAs per SM)
-    for (int h = 0; h < 2 && run; h++) {
-    if (t == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");   // after the first half's TMEM reads
-        const uint32_t idesc = (2u << 4) | ((uint32_t)(NS >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-        const uint32_t aa = smem_u32(sA), ac = smem_u32(sC);
+        for (int c = 0; c < LH; c++) v[c] = ok && (!half || LH + c < L) ? (u32)__ldg(src + c * a.plane) : 0u;
+        vneg = ok && __ldg(a.m + b * a.sb + r * a.sr + k * a.sk + (int64_t)(L - 1) * a.plane) < 0;
+    };
+    // reduction: lane = element (row lane / 16 of the warp's two, column lane % 16); chunk halves by warp / 4
+    const int quad = warp & 3, part = warp >> 2, q4 = lane & 3;
+    const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
+    const u32 sel1 = q4 & 2 ? 0x3276u : 0x5410u, sel2 = q4 & 1 ? 0x3715u : 0x6240u;
+    const int N1 = (NS / 2 + 15) / 16 * 16;              // chunk columns: N1 and NS - N1 of each tile of the constant
+    const uint64_t da0 = umma_desc(smem_u32(sA), 128 * 16, 128), dc0 = umma_desc(smem_u32(sC), NS * 16, 128);
+    auto chunk_n = [&](int q) { return q & 1 ? NS - N1 : N1; };
+    auto chunk_j = [&](int q) { return ((q >> 1) * NS + (q & 1 ? N1 : 0)) / 4; };
+    auto issue = [&](int q) {                            // thread 0
+        const int n = chunk_n(q);
+        const uint32_t idesc = (2u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint64_t dc = dc0 + (uint64_t)(((q >> 1) * NS * Ks + (q & 1 ? N1 * 16 : 0)) >> 4);
         for (int kk = 0; kk < Ks / 32; kk++) {
-            uint64_t da = umma_desc(aa + kk * 2 * (128 * 16), 128 * 16, 128);
-            uint64_t db = umma_desc(ac + h * NS * Ks + kk * 2 * (NS * 16), NS * 16, 128);
-            uint32_t acc = kk > 0 ? 1u : 0u;
+            const uint32_t acc = kk > 0 ? 1u : 0u;
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "setp.ne.b32 p, %4, 0;\n\t"
                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                ::"r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+                ::"r"(tmem + 128u * (q & 1)), "l"(da0 + (uint64_t)(kk * 256)), "l"(dc + (uint64_t)(kk * 2 * NS)), "r"(idesc),
+                  "r"(acc) : "memory");
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                     ::"r"(smem_u32(&bar_mma)) : "memory");
-    }
-    mma_h = h;
-    if (!mbar_wait(&bar_mma, h, kWaitLimit)) atomicExch(&fail_sh, 2);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    __syncthreads();
-    run = fail_sh == 0;
-    if (run) {
-        // epilogue: element e = t; residues of 4 primes per 16-column chunk, primes of this half
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-        const bool neg = neg_sh[t];
-        const int rr = t / 16, kk = t % 16;
-        const int jlo = h * (NS / 4), jhi = (h + 1) * (NS / 4) < np ? (h + 1) * (NS / 4) : np;
-        for (int j0 = jlo; j0 < jhi; j0 += 4) {
-            uint32_t d[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
-                  "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
-                : "r"(taddr + (uint32_t)(4 * j0 - h * NS)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                     ::"r"(smem_u32(&bar_mma[q & 1])) : "memory");
+    };
+    uint32_t phase = 0;                                  // bit x: commits waited for so far on buffer x, modulo 2
+    uint32_t out_mma = 0;                                // thread 0: buffers whose commit is not yet waited for (failure drain)
+    if ((int64_t)blockIdx.x < items && run) load(blockIdx.x);
+    for (int64_t item = blockIdx.x; item < items && run; item += gridDim.x) {
+        const int64_t b = item / tiles, tile = item % tiles;
+        const int64_t r0 = (tile / ktiles) * 8, k0 = (tile % ktiles) * 16;
+        const u32 flip = vneg ? 0xFFFFFFFFu : 0u;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int j = j0 + q;
-                if (j >= np) break;
-                uint64_t v = (uint64_t)d[4 * q] + ((uint64_t)d[4 * q + 1] << 8) + ((uint64_t)d[4 * q + 2] << 16) +
-                             ((uint64_t)d[4 * q + 3] << 24);
-                const uint32_t p = __ldg(tb.p + j);
-                uint32_t r = barrett(v, p, __ldg(tb.mu + j));
-                if (neg && r) r = p - r;
+        for (int c = 0; c < LH; c++)
+            if (!half || LH + c < L) v[c] ^= flip;
 #pragma unroll
-                for (int s = 0; s < 4; s++) sD[((j * 4 + s) * 8 + rr) * 16 + kk] = (uint8_t)(r >> (8 * s));
+        for (int c = 0; c < LH / 4; c++)
+            if (half == 0 || LH / 4 + c < Ks / 16)
+                *reinterpret_cast<uint4*>(sA + (size_t)((half ? LH / 4 : 0) + c) * 2048 + (le >> 3) * 128 + (le & 7) * 16) =
+                    make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+        if (half) {
+            for (int c = LH / 2; c < Ks / 16; c++)
+                *reinterpret_cast<uint4*>(sA + (size_t)c * 2048 + (le >> 3) * 128 + (le & 7) * 16) = make_uint4(0, 0, 0, 0);
+            neg_sh[le] = vneg;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // generic-proxy writes -> tensor core
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        if (t == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int q = 0; q < 2; q++)
+                if (chunk_n(q) > 0 && chunk_j(q) < np) { issue(q); out_mma |= 1u << q; }
+        }
+        if (item + gridDim.x < items) load(item + gridDim.x);
+        const u32 neg = neg_sh[quad * 32 + lane];
+        const int64_t row = 4 * (r0 + quad * 2 + (lane >> 4)) + q4;
+        const bool store = row < 4 * a.Rp;
+        uint8_t* obase = a.out + (size_t)b * a.mat_bytes + tiled_offset(row, k0, a.TR, a.Kp) + (lane & 12);
+        const size_t ostep = (size_t)a.nb * a.mat_bytes;
+#pragma unroll 1
+        for (int q = 0; q < 4; q++) {
+            const int jlo = chunk_j(q), n = chunk_n(q);
+            if (n == 0 || jlo >= np) continue;
+            if (!mbar_wait(&bar_mma[q & 1], (phase >> (q & 1)) & 1u, kWaitLimit)) atomicExch(&fail_sh, 2);
+            else out_mma &= ~(1u << (q & 1));
+            phase ^= 1u << (q & 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int jn = jlo + n / 4 < np ? n / 4 : np - jlo;
+            for (int g = part; 4 * g < jn; g += 2) {
+                uint32_t d[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                    : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
+                      "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
+                    : "r"(taddr + (uint32_t)(128 * (q & 1) + 16 * g)));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const int j = jlo + 4 * g;
+                uint2 pt[4];
+                uint32_t r[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) pt[u] = tab[j + u];
+                if (near) {                              // d < 2^23.6: both halves fit 32 bits
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        r[u] = mod_near48(widen16(d[4 * u + 3] * 256u + d[4 * u + 2], d[4 * u + 1] * 256u + d[4 * u] + neg),
+                                          pt[u].x, pt[u].y);
+                } else {
+#pragma unroll 1
+                    for (int u = 0; u < 4; u++) {
+                        const uint64_t x = u == 0 ? widen16(d[3] * 256u + d[2], d[1] * 256u + d[0] + neg)
+                                         : u == 1 ? widen16(d[7] * 256u + d[6], d[5] * 256u + d[4] + neg)
+                                         : u == 2 ? widen16(d[11] * 256u + d[10], d[9] * 256u + d[8] + neg)
+                                                  : widen16(d[15] * 256u + d[14], d[13] * 256u + d[12] + neg);
+                        const uint32_t m = barrett(x, tab[j + u].x, __ldg(tb.mu + (j + u < np ? j + u : 0)));
+                        if (u == 0) r[0] = m;
+                        else if (u == 1) r[1] = m;
+                        else if (u == 2) r[2] = m;
+                        else r[3] = m;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) r[u] = neg ? pt[u].x - r[u] : r[u];   // p for a zero residue: as good
+                u32 w[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) w[u] = __byte_perm(r[u], __shfl_xor_sync(0xFFFFFFFFu, r[u], 2), sel1);
+#pragma unroll
+                for (int u = 0; u < 4; u++) w[u] = __byte_perm(w[u], __shfl_xor_sync(0xFFFFFFFFu, w[u], 1), sel2);
+                uint8_t* o = obase + (size_t)j * ostep;
+#pragma unroll
+                for (int u = 0; u < 4; u++, o += ostep)
+                    if (store && j + u < np) *reinterpret_cast<u32*>(o) = w[u];
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncthreads();                              // the buffer is read out
+            if (t == 0 && q < 2 && chunk_n(q + 2) > 0 && chunk_j(q + 2) < np) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                issue(q + 2);
+                out_mma |= 1u << q;
             }
         }
+        run = fail_sh == 0;
+        __syncthreads();                                  // fail_sh is read before the next tile's waits
     }
-    mma_h = h;
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();                                      // TMEM read out before the second half's MMAs
-    }
-    __syncthreads();
-    if (run) {
-        // 16-byte chunks: (prime j, digit s, row rr) -> row 4 (r0 + rr) + s, columns k0 .. k0 + 15
-        for (int c = t; c < np * 32; c += 128) {
-            const int rr = c % 8, s = (c / 8) % 4, j = c / 32;
-            const int64_t r = r0 + rr;
-            if (r >= a.Rp) continue;
-            uint4 w = *reinterpret_cast<const uint4*>(sD + (size_t)c * 16);
-            *reinterpret_cast<uint4*>(a.out + ((size_t)j * a.nb + b) * a.mat_bytes + tiled_offset(4 * r + s, k0, a.TR, a.Kp)) = w;
-        }
-    }
-    __syncthreads();                                      // sD and neg_sh are rewritten by the next tile
-    }
-    if (t == 0 && fail_sh) {
+    if (t == 0 && fail_sh) {                              // bounded drain of our own copy and MMAs
         if (!mbar_wait(&bar_load, 0, kWaitLimit)) fail_sh = 3;
-        else if (fail_sh == 2 && !mbar_wait(&bar_mma, mma_h, kWaitLimit)) fail_sh = 4;
+        for (int q = 0; q < 2; q++)
+            if ((out_mma >> q & 1u) && !mbar_wait(&bar_mma[q], ((phase >> q) & 1u) ^ 1u, kWaitLimit)) fail_sh = 4;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
     }
     if (t == 0 && fail_sh) atomicExch(a.err, fail_sh);
 }
@@ -909,7 +1013,7 @@ template <int L>
 int RnsLaunch<L>::split_mma(const RnsSplit& a, const RnsTables& tb, cudaStream_t st) {
     static unsigned long long configured = 0;            // devices whose shared-memory limit is raised
     const unsigned long long dbit = device_bit();
-    const int smem = 128 * a.Ks + 2 * a.NS * a.Ks + tb.np * 512;
+    const int smem = rns_split_smem(a.Ks, a.NS, tb.np);
     if (!(configured & dbit) || !dbit) {
         int rc = (int)cudaFuncSetAttribute(k_rns_split_mma<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRnsSmemCap);
         if (rc) return rc;
@@ -925,7 +1029,7 @@ int RnsLaunch<L>::split_mma(const RnsSplit& a, const RnsTables& tb, cudaStream_t
     }
     const int64_t items = (a.Kp / 16) * ((a.Rp + 7) / 8) * a.nb;
     const int64_t ctas = items < 2 * (int64_t)sms ? items : 2 * (int64_t)sms;   // two CTAs per SM, persistent
-    k_rns_split_mma<L><<<(unsigned)ctas, 128, smem, st>>>(a, tb);
+    k_rns_split_mma<L><<<(unsigned)ctas, 256, smem, st>>>(a, tb);
     return (int)cudaGetLastError();
 }
 

@@ -162,7 +162,7 @@ class Recursion:
         Kp = -(-Kc // 32) * 32
         table = self._cauchy_table()
         c_rows = Mr >= N                                           # C on the 128 TMEM lanes
-        TN = min(256, -(-4 * (N if c_rows else Mr) // 16) * 16)
+        TN = rns.column_tile(N if c_rows else Mr)
         TRc = 128 if c_rows else TN
         Rp_c = -(-Mr // (TRc // 4)) * (TRc // 4)
         c_mat = 4 * Rp_c * Kp

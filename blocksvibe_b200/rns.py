@@ -187,6 +187,13 @@ def _round_up(x, m):
     return -(-x // m) * m
 
 
+def column_tile(rows):
+    """digit rows per column tile of the residue product: at most 256, evenly sized (132 rows, 528 digit rows: three
+    tiles of 176, not of 256 with the last one nearly empty)"""
+    n = 4 * max(rows, 1)
+    return _round_up(-(-n // -(-n // 256)), 16)
+
+
 SPLIT = "tensor"          # "tensor": residue digits on the tensor cores; "cuda": on the CUDA cores
 
 # int8 multiply-accumulates issued to the tensor cores by the residue products since the last reset (the work
@@ -233,7 +240,7 @@ def gemm_aligned_rns(Aal, Bal, crt="tensor", lanes=None):
     else:
         xs, ys, out_i, out_l = b_rows, a_rows, 1, N
     NL = ys["R"]
-    TN = min(256, _round_up(4 * NL, 16))
+    TN = column_tile(NL)
     X, x_mat, _ = _split(tb, xs["m"], xs["plane"], nb, xs["R"], K, xs["sb"], xs["sr"], xs["sk"], Kp, 128, stream)
     Y, y_mat, Rp_y = _split(tb, ys["m"], ys["plane"], nb, NL, K, ys["sb"], ys["sr"], ys["sk"], Kp, TN, stream)
     n = nb * M * N
