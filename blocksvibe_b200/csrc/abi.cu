@@ -139,7 +139,19 @@ int b3d_moments_flush(int L, const int32_t* ym, const int64_t* ye, int64_t yplan
     if ((Lout != L && Lout != L + 4) || !b3d_supported_limbs(Lout))
         return fail(B3D_E_ARG, "b3d_moments_flush: Lout must be L or L + 4 (compiled)");
     B3D_DISPATCH(L, cuda_status(LX::moments_flush(ym, ye, yplane, row_shift, m0, W, rows, N, R1, nk, nkb, NN, KW,
-                                                 accumulate, Lout, mm, me, mplane, as_stream(stream)), "b3d_moments_flush"));
+                                                 accumulate, Lout, mm, me, mplane, false, as_stream(stream)), "b3d_moments_flush"));
+}
+
+int b3d_moments_flush_mma(int L, const int32_t* ym, const int64_t* ye, int64_t yplane, const int64_t* row_shift, int64_t m0,
+                          int W, int64_t rows, int64_t N, int R1, const uint32_t* nk, const int32_t* nkb, int NN, int KW,
+                          int accumulate, int Lout, int32_t* mm, int64_t* me, int64_t mplane, int* err, void* stream) {
+    if (!nonneg(rows) || !nonneg(N) || !nonneg(m0) || W < 0 || R1 < 1 || R1 > 32 || NN < 1 || KW < 1 || KW > 12)
+        return fail(B3D_E_ARG, "b3d_moments_flush_mma: invalid size (1 <= R + 1 <= 32, 1 <= KW <= 12)");
+    if ((Lout != L && Lout != L + 4) || !b3d_supported_limbs(Lout))
+        return fail(B3D_E_ARG, "b3d_moments_flush_mma: Lout must be L or L + 4 (compiled)");
+    if (!err) return fail(B3D_E_ARG, "b3d_moments_flush_mma: no error flag");
+    b3d::FlushMmaArgs a{ym, ye, yplane, row_shift, m0, rows, N, W, R1, NN, KW, nk, nkb, mm, me, mplane, err};
+    B3D_DISPATCH_FLUSH(L, cuda_status(MX::flush(a, accumulate, Lout, as_stream(stream)), "b3d_moments_flush_mma"));
 }
 
 int b3d_resize(int L, const int32_t* m, const int64_t* e, int64_t plane, int64_t n, int Lout, int32_t* om, int64_t* oe,

@@ -6,10 +6,11 @@
 #include "rns.cuh"
 #include "cauchy_rns.cuh"
 #include "cauchy_fp.cuh"
+#include "moments_mma.cuh"
 
 namespace b3d {
 #define B3D_DECL(L) extern template struct Launch<L>; extern template struct RnsLaunch<L>; extern template struct CauchyRnsLaunch<L>; \
-    extern template struct CauchyFpLaunch<L>;
+    extern template struct CauchyFpLaunch<L>; extern template struct FlushMmaLaunch<L>;
 B3D_FOR_EACH_L(B3D_DECL)
 #undef B3D_DECL
 
@@ -68,6 +69,22 @@ int cauchy_digits_launch(const CauchyLevel& lv, const uint32_t* table, int64_t d
         case 38: { using FX = b3d::CauchyFpLaunch<38>; return CALL; }\
         case 46: { using FX = b3d::CauchyFpLaunch<46>; return CALL; }\
         case 42: { using FX = b3d::CauchyFpLaunch<42>; return CALL; }         \
+        default: return b3d::fail(B3D_E_LIMBS, "no kernels compiled for L = " + std::to_string(L)); \
+    }
+
+#define B3D_DISPATCH_FLUSH(L, CALL)                                           \
+    switch (L) {                                                               \
+        case 6: { using MX = b3d::FlushMmaLaunch<6>; return CALL; }           \
+        case 10: { using MX = b3d::FlushMmaLaunch<10>; return CALL; }         \
+        case 18: { using MX = b3d::FlushMmaLaunch<18>; return CALL; }         \
+        case 26: { using MX = b3d::FlushMmaLaunch<26>; return CALL; }         \
+        case 30: { using MX = b3d::FlushMmaLaunch<30>; return CALL; }         \
+        case 34: { using MX = b3d::FlushMmaLaunch<34>; return CALL; }         \
+        case 14: { using MX = b3d::FlushMmaLaunch<14>; return CALL; }\
+        case 22: { using MX = b3d::FlushMmaLaunch<22>; return CALL; }\
+        case 38: { using MX = b3d::FlushMmaLaunch<38>; return CALL; }\
+        case 46: { using MX = b3d::FlushMmaLaunch<46>; return CALL; }\
+        case 42: { using MX = b3d::FlushMmaLaunch<42>; return CALL; }         \
         default: return b3d::fail(B3D_E_LIMBS, "no kernels compiled for L = " + std::to_string(L)); \
     }
 

@@ -6,6 +6,7 @@
 #include "cauchy_fp.cuh"
 #include "decimal.cuh"
 #include "pole_mma.cuh"
+#include "moments_mma.cuh"
 
 #ifndef B3D_L
 #error "compile with -DB3D_L=<limbs>"
@@ -16,5 +17,6 @@ template struct Launch<B3D_L>;
 template struct RnsLaunch<B3D_L>;
 template struct CauchyRnsLaunch<B3D_L>;
 template struct CauchyFpLaunch<B3D_L>;
+template struct FlushMmaLaunch<B3D_L>;
 template struct DecimalLaunch<B3D_L>;
 }

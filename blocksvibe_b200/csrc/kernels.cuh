@@ -890,7 +890,7 @@ template <int L, int LO, int KW, bool ACCUMULATE>
 __global__ void __launch_bounds__(kFlushThreads) k_moments_flush(const int32_t* __restrict__ ym, const i64* __restrict__ ye,
                           i64 yplane, const i64* __restrict__ row_shift, i64 m0, int W, i64 rows, i64 N, int R1,
                           const u32* __restrict__ nk, const int32_t* __restrict__ nkb, int NN,
-                          int32_t* __restrict__ mm, i64* __restrict__ me, i64 mplane) {
+                          int32_t* __restrict__ mm, i64* __restrict__ me, i64 mplane, bool zero_rows) {
     constexpr int NB = nb_bits(L);                       // staged terms: L limbs; moments: LO limbs
     constexpr int ACC = LO + 3;
     constexpr int NP = L + KW + 1;                       // |Y| n^k, k within a chunk: n^k0 < 2^(32 KW), n^3 < 2^32
@@ -899,6 +899,7 @@ __global__ void __launch_bounds__(kFlushThreads) k_moments_flush(const int32_t* 
     if (item >= rows * N) return;
     const i64 row = item / N, c = item - row * N;
     const i64 sh = row_shift[row];
+    if (zero_rows && m0 + sh > 0) return;                // only the rows with n = 0 in the window
     u32* acc = flush_acc + threadIdx.x;
     for (int k0 = 0; k0 < R1; k0 += kFlushKC) {
         const int kc = R1 - k0 < kFlushKC ? R1 - k0 : kFlushKC;
@@ -1055,7 +1056,7 @@ struct Launch {
                              int32_t* ym, i64* ye, i64 yplane, cudaStream_t st);
     static int moments_flush(const int32_t* ym, const i64* ye, i64 yplane, const i64* row_shift, i64 m0, int W, i64 rows,
                              i64 N, int R1, const u32* nk, const int32_t* nkb, int NN, int KW, int accumulate, int LO,
-                             int32_t* mm, i64* me, i64 mplane, cudaStream_t st);
+                             int32_t* mm, i64* me, i64 mplane, bool zero_rows, cudaStream_t st);
     static int resize(const int32_t* m, const i64* e, i64 plane, i64 n, int LO, int32_t* om, i64* oe, i64 oplane,
                       cudaStream_t st);
 };
@@ -1191,7 +1192,7 @@ int Launch<L>::moments_stage(const int32_t* rm, const i64* re, i64 rplane, const
 template <int L>
 int Launch<L>::moments_flush(const int32_t* ym, const i64* ye, i64 yplane, const i64* row_shift, i64 m0, int W, i64 rows,
                              i64 N, int R1, const u32* nk, const int32_t* nkb, int NN, int KW, int accumulate, int LO,
-                             int32_t* mm, i64* me, i64 mplane, cudaStream_t st) {
+                             int32_t* mm, i64* me, i64 mplane, bool zero_rows, cudaStream_t st) {
     const i64 items = rows * N;
     if (items == 0 || W == 0) return 0;
     const unsigned grid = (unsigned)((items + kFlushThreads - 1) / kFlushThreads);
@@ -1206,7 +1207,7 @@ int Launch<L>::moments_flush(const int32_t* ym, const i64* ye, i64 yplane, const
             opted |= dbit;                                                                                       \
         }                                                                                                    \
         k_moments_flush<L, LOC, KWC, AC><<<grid, kFlushThreads, smem, st>>>(ym, ye, yplane, row_shift, m0, W, rows, N, R1, \
-                                                                            nk, nkb, NN, mm, me, mplane);    \
+                                                                            nk, nkb, NN, mm, me, mplane, zero_rows); \
     } while (0)
 #define B3D_FLUSH_KW(LOC) \
     if (KW <= 2) { if (accumulate) B3D_FLUSH(LOC, 2, true); else B3D_FLUSH(LOC, 2, false); } \

@@ -165,6 +165,7 @@ class Derivs:
         # index tensors of finish_iter, built once (no host-to-device copies while a CUDA graph is captured)
         self._jidx = torch.tensor([(tj - tj12 % 2) // 2 for tj in self.tjs], device=self.device)
         self._orders = {}
+        self.err = torch.zeros(1, dtype=torch.int32, device=self.device)   # bounded-wait expiries of the flush
         self._acache = {}                  # row-aligned constant GEMM operands (shared by the for_order copies)
 
     # ------------------------------------------------------------ moment bookkeeping per level
@@ -351,13 +352,20 @@ class Derivs:
         R1 = self.R + 1
         nk = self._nk[:R1].contiguous()
         nkb = self._nkb[:R1].contiguous()
-        _lib.call("b3d_moments_flush", self.L, p(self._stage.m), p(self._stage.e), self._stage.m.stride(0),
+        _lib.call("b3d_moments_flush_mma", self.L, p(self._stage.m), p(self._stage.e), self._stage.m.stride(0),
                   p(self._row_shift), self._m0, W, rows, self.N, R1, p(nk), p(nkb), self.plan.order + 1, self._KW,
-                  int(self._flushes > 0), self.Ld, p(self.mom.m), p(self.mom.e), self.mom.m.stride(0),
+                  int(self._flushes > 0), self.Ld, p(self.mom.m), p(self.mom.e), self.mom.m.stride(0), p(self.err),
                   torch.cuda.current_stream(self.device).cuda_stream)
         self._flushes += 1
         self._last = None
         self._stage.e.fill_(mpf.EZ)                      # entries a level does not write read as zero
+
+    def check_errors(self):
+        """raise B3DError if the flush gave up a bounded wait (synchronises the device)"""
+        code = int(self.err.item())
+        if code:
+            self.err.zero_()
+            raise _lib.B3DError(f"moments flush: the tensor-core kernel did not complete (code {code})")
 
     # ------------------------------------------------------------ final GEMMs
     def finish(self, h_inf, chunk=None):

@@ -128,6 +128,14 @@ int b3d_moments_flush(int L, const int32_t* ym, const int64_t* ye, int64_t yplan
                       int W, int64_t rows, int64_t N, int R1, const uint32_t* nk, const int32_t* nkb, int NN, int KW,
                       int accumulate, int Lout, int32_t* mm, int64_t* me, int64_t mplane, void* stream);
 
+/* The same flush with the sums as INT8 tensor-core GEMMs of balanced base-256 digits (replaces the windowed momflush of
+ * the reference, derivatives.py:124-188, like b3d_moments_flush) where the window has enough levels and the integers fit
+ * one tile, b3d_moments_flush's kernel otherwise.  err: a device int set nonzero if a bounded wait of the kernel expired or
+ * the table does not hold n^k (results then incomplete). */
+int b3d_moments_flush_mma(int L, const int32_t* ym, const int64_t* ye, int64_t yplane, const int64_t* row_shift, int64_t m0,
+                          int W, int64_t rows, int64_t N, int R1, const uint32_t* nk, const int32_t* nkb, int NN, int KW,
+                          int accumulate, int Lout, int32_t* mm, int64_t* me, int64_t mplane, int* err, void* stream);
+
 /* Change of limb count of n numbers, Lout = L or L +- 4: widening is exact, narrowing rounds once (half away from
  * zero).  The derivative stages run with more limbs than the recursion where their sums cancel (the drop-in's
  * choice; no counterpart in the reference, whose stages share one limb count). */
