@@ -27,7 +27,7 @@
 #include <cmath>
 
 #include "kernels.cuh"
-#include "rns.cuh"
+#include "pole_mma.cuh"
 
 namespace b3d {
 
@@ -95,16 +95,6 @@ inline bool flush_mma_geom(int LO, int W, int R1, int NN, int KW, FlushGeom* out
 }
 
 #ifdef B3D_DEFINE_LAUNCH
-// sixteen TMEM columns of a warp's lanes (not waited for)
-__device__ __forceinline__ void tmem_ld16(int* d, uint32_t addr) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]),
-          "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
-        : "r"(addr));
-}
-
 // bit i of a 64-bit mask: the predicate of limb i, two limbs per lane (i = lane, lane + 32)
 __device__ __forceinline__ u64 ballot2(bool lo, bool hi) {
     return (u64)__ballot_sync(0xFFFFFFFFu, lo) | ((u64)__ballot_sync(0xFFFFFFFFu, hi) << 32);
@@ -301,16 +291,14 @@ __global__ void __launch_bounds__(kFlushMmaThreads, 2) k_moments_flush_mma(Flush
                 i64 cy = 0;
                 const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16);
                 const int i1 = qt == NX - 1 || (qt + 1) * h > g.VW ? g.VW : (qt + 1) * h;
-                for (int i = qt * h; i < i1; i += 8) {
-                    int d[32];
+                for (int i = qt * h; i < i1; i += 4) {
+                    uint32_t d[16];
                     tmem_ld16(d, ta + (uint32_t)(4 * i));
-                    const bool two = i + 4 < i1;
-                    if (two) tmem_ld16(d + 16, ta + (uint32_t)(4 * i + 16));
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        if (u >= 4 && !two) break;
-                        const i64 x = (i64)d[4 * u] + (i64)d[4 * u + 1] * 256 + ((i64)d[4 * u + 2] + (i64)d[4 * u + 3] * 256) * 65536;
+                    for (int u = 0; u < 4; u++) {
+                        const i64 x = (i64)(int)d[4 * u] + (i64)(int)d[4 * u + 1] * 256 +
+                                      ((i64)(int)d[4 * u + 2] + (i64)(int)d[4 * u + 3] * 256) * 65536;
                         const i64 s = x + cy;
                         if (r < g.Mrows) v[(i + u) * RS] = (u32)s;
                         cy = s >> 32;

@@ -14,24 +14,26 @@
 // canonical no-swizzle K-major descriptor with LBO = 256 (next K chunk = 16 offsets on) and SBO = 128
 // (next 8 rows = 8 offsets on).  |D| <= S 4 L 2^14 < 2^31: no wrap.
 //
-// Positions below P0 (a multiple of 16; zero when two 128-lane tiles cover the whole product) are not
-// computed.  Their sum is below 2^(8 P0 + 17) in magnitude, far under the rounding point of the result;
-// the rounding is kept where no value that close rounds differently (the test of round_safe), and where it
-// is not (exact cancellation, a sum at a rounding midpoint) the thread adds the missing positions exactly
-// from the digits still in shared memory.
+// Positions below P0 (a multiple of 16) are not computed: their sum is below 2^(8 P0 + 17) in magnitude, at least 96
+// bits under the rounding point of a sum as long as the operands allow.  The rounding is kept where no value that close
+// rounds differently, and where it is not (deep cancellation, a sum at a rounding midpoint) the thread forms the exact sum
+// from the operands in memory.
 //
-// One CTA (128 threads) per (task, column chunk of NC <= 32 columns), persistent over the work list:
-//   1. column exponents, then the aligned X digits into the K-major B operand (16-byte stores);
-//   2. per row i: the padded digit strings of c_ij (the next row's constants load meanwhile), the Hankel
-//      windows (four per thread step, byte permutations of five words, stored in a rotated order that
-//      keeps the stores free of bank conflicts), fence.proxy.async, one thread issues MT x S x U / 32 MMAs
-//      (M = 128, N = NC, K = 32), commits to an mbarrier and waits for it;
-//   3. per tile of 128 positions, tcgen05.ld of the accumulators, transposed through shared memory
-//      (D[n][p]); the carry chain (64-bit multiply-adds of four positions per limb) in segments of eight
-//      limbs, one per warp and a lane per column, into a shared-memory limb column; then one header thread
-//      per column joins the segments' carries, checks the rounding and decides it (top limb, shift, carry
-//      and sign extents), and all threads write the rounded limbs, a lane per column (runs of consecutive
-//      outputs in each limb plane).
+// One CTA (160 threads, three per SM) works through (task, column chunk of NC <= 32 columns) items.  Four front warps, per
+// item: column exponents, the aligned X digits into the K-major B operand (16-byte stores); per row i: the padded digit
+// strings of c_ij (the next row's constants load meanwhile), the Hankel windows (four per thread step, byte permutations
+// of five words, stored in a rotated order that keeps the stores free of bank conflicts), one thread issues the MMAs (M =
+// 128, N = NC, K = 32: two 16-digit chunks, the second of which may start the next entry, so that entries are not padded to
+// 32 digits); then the accumulators go transposed (D[n][p]) into a shared-memory slot.  A back warp, a lane per column, takes
+// the slot: the limbs of the sum by one carry chain in registers (the slot is free again), sign, one rounding, coalesced
+// stores, while the front warps multiply the next row.  Slot and rows pass by mbarriers.
+//
+// What bounds it: latency; the MMAs (38 clocks each, their 128-row A operand through shared memory) keep the tensor path
+// busy for a good half of the time at S = 5, L = 34.  Per 1024-bit task (134,316 tasks of 30 columns, both stages): 18.8 ms;
+// two CTAs of four front and four back warps 22.7 (26.9 and 24.8 with the next item's operands prefetched or preloaded:
+// registers spill), TMEM read 32 columns at a time 26.5 (through local memory).  The form before handled a row in four warps
+// by turns (windows, MMAs, carry segments, one header thread per column, limbs by run-time offsets) with all 256 positions:
+// some 8,000 warp instructions and 10,000 clocks of a CTA per row, 27.8 ms.
 // Every mbarrier wait is bounded; on expiry the CTA records an error code, waits (bounded) for its own MMAs,
 // frees its TMEM and returns.
 #pragma once
@@ -46,24 +48,27 @@ template <int L>
 struct PoleMmaGeom {
     static constexpr int NB = nb_bits(L);
     static constexpr int D = 4 * L;                                 // digits of a number
-    static constexpr int U = 32 * ((D + 31) / 32);                  // digits per entry along K (MMA K step 32)
+    static constexpr int U = 16 * ((D + 15) / 16);                  // digits per entry along K (chunks of 16)
+    static constexpr int NCH = U / 16;
     static constexpr int p0_for(int mt) {
         return 8 * L - 1 - 128 * mt <= 0 ? 0 : 16 * ((8 * L - 1 - 128 * mt + 15) / 16);
     }
     // one tile of 128 positions where the dropped part stays 160 bits below the result's rounding point
     static constexpr int MT = (8 * p0_for(1) + 17 <= NB - 160) ? 1 : 2;
-    static constexpr int P0 = p0_for(MT);                            // first position computed
-    static constexpr int NWIN = 128 * MT + U - 16;                  // Hankel windows per entry (a multiple of 16)
+    // first position computed: as high as leaves 96 bits below the rounding point
+    static constexpr int p0_high() { return NB - 96 - 17 < 128 ? 0 : 16 * ((NB - 96 - 17) / 128); }
+    static constexpr int P0 = p0_high() > p0_for(MT) ? p0_high() : p0_for(MT);
+    static constexpr int NP = 8 * L - P0;                           // positions computed (a multiple of 16)
+    static constexpr int NWIN = NP + U - 16;                        // Hankel windows per entry (a multiple of 16)
     static constexpr int FAM = 16 * NWIN;                           // bytes of one entry's windows
-    static constexpr int PADB = U;                                  // zero bytes before a digit string
-    static constexpr int CW = (P0 + 128 * MT + 2 * U) / 4 + 2;      // words of a padded digit string
-    static constexpr int NW = 2 * L + 2;                            // accumulator limbs
-    static constexpr int EW = P0 / 4 + 1;                           // error of the truncated sum < 2^(32 EW)
-    static constexpr int VW = 32 * MT;                              // 4-position words per column
-    static constexpr int DS = 128 + 4;                              // words per transposed column of a tile (16-byte rows)
-    static_assert(8 * P0 + 17 <= NB - 160, "two tiles must reach the rounding point");
-    static_assert(U / 4 + L <= CW, "digit string inside its padded buffer");
-    static_assert(NWIN % 4 == 0 && (P0 + 1) % 4 == 1, "window groups start one byte after a word");
+    static constexpr int SPAN = 16 * (128 * MT + U + 16);            // bytes the MMAs may touch from an entry's windows on
+    static constexpr int PADB = U - P0;                             // zero bytes before a digit string (negative: it starts P0 - U in)
+    static constexpr int CW = (NP + U) / 4 + 2;                     // words of a padded digit string from byte P0 on
+    static constexpr int NPW = NP / 4;                              // limbs of a sum from position P0 up
+    static constexpr int DS = NP + 4;                               // words per transposed column (16-byte rows)
+    static_assert(8 * P0 + 17 <= NB - 64 && NP > 0 && NP <= 128 * MT && NP % 16 == 0, "tiles must reach the rounding point");
+    static_assert(PADB >= 0 && PADB % 4 == 0 && PADB / 4 + L <= CW, "digit string inside its padded buffer");
+    static_assert(NWIN % 4 == 0, "window groups start one byte after a word");
 };
 
 struct PoleMmaArgs {
@@ -80,30 +85,33 @@ struct PoleMmaArgs {
     int* err;                                       // device error flag (0 = ok)
 };
 
-constexpr int kPoleMmaThreads = 128;
+constexpr int kPoleMmaThreads = 160;                            // four front warps, one back warp
 constexpr int kPoleMmaMaxS = 8;
 constexpr int kPoleMmaMaxNC = 32;
 
 __host__ __device__ constexpr size_t pm_align(size_t x) { return (x + 127) & ~size_t(127); }
 
-// dynamic shared memory: B operand | Hankel windows, reused by the transposed accumulators and the limb
-// columns once the MMAs are done | padded digit strings of two rows (this one and the next) | column exponents
+// dynamic shared memory: B operand (a zero chunk after an odd number of them) | Hankel windows | padded digit strings of two
+// rows (this one and the next) | a slot of transposed accumulators | column exponents of the item and of the slot (and the
+// slot's row exponent) | A descriptors of the K steps
 template <int L>
 struct PoleMmaSmem {
     using G = PoleMmaGeom<L>;
-    static __host__ __device__ size_t bop(int S, int NC) { return pm_align((size_t)S * G::U * NC); }
-    static __host__ __device__ size_t dbuf(int NC) { return (size_t)NC * G::DS * 4; }
-    static __host__ __device__ size_t hank(int S, int NC) {
-        const size_t h = (size_t)S * G::FAM, v = dbuf(NC) + (size_t)G::NW * (NC + 1) * 4;
-        return pm_align(h > v ? h : v);
-    }
+    static __host__ __device__ int steps(int S) { return (S * G::NCH + 1) / 2; }
+    static __host__ __device__ size_t bop(int S, int NC) { return pm_align((size_t)steps(S) * 32 * NC); }
+    static __host__ __device__ size_t hank(int S) { return pm_align((size_t)S * G::FAM); }
     static __host__ __device__ size_t cdig(int S) { return pm_align((size_t)2 * S * G::CW * 4); }   // two rows
+    static __host__ __device__ size_t slot(int NC) { return pm_align((size_t)NC * G::DS * 4); }
     static __host__ __device__ size_t total(int S, int NC) {
-        return bop(S, NC) + hank(S, NC) + cdig(S) + pm_align((size_t)NC * 8);
+        const size_t t = bop(S, NC) + hank(S) + cdig(S) + slot(NC) + 2 * (kPoleMmaMaxNC + 1) * 8 + (size_t)steps(S) * 8;
+        const size_t read = bop(S, NC) + (size_t)(S - 1) * G::FAM + G::SPAN;
+        return pm_align(t > read ? t : read);
     }
 };
 
 // v (two's complement, L words) -> balanced base-256 digits, four per word (little-endian bytes, as s8)
+template <int L> B3D_CX bool P0_exact() { return PoleMmaGeom<L>::P0 == 0; }      // nothing is dropped
+
 template <int L> __device__ __forceinline__ void to_balanced(u32 (&v)[L]) {
     u32 c = 0;
 #pragma unroll
@@ -113,8 +121,6 @@ template <int L> __device__ __forceinline__ void to_balanced(u32 (&v)[L]) {
         v[k] = (u32)s ^ 0x80808080u;
     }
 }
-
-__device__ __forceinline__ int sbyte(const uint8_t* p, int i) { return (int)(int8_t)p[i]; }
 
 // Offsets inside a task's (S, S, B) block: X entry (j, column n) at coff(n) + j * jst, output (i, column n) at
 // coff(n) + i * jst, with n = a B + k in stage 1 (X[a, j, k], Y[a, i, k]) and n = b0 B + k in stage 2
@@ -126,210 +132,158 @@ __device__ __forceinline__ int pm_coff(const PoleMmaArgs& a, int n) {
 
 __device__ __forceinline__ int pm_jst(const PoleMmaArgs& a) { return a.stage == 1 ? (int)a.B : a.S * (int)a.B; }
 
-template <int L> __device__ __forceinline__ void pm_store_zero(const PoleMmaArgs& a, i64 o) {
-#pragma unroll
-    for (int k = 0; k < L; k++) a.om[k * a.oplane + o] = 0;
-    a.oe[o] = EZ;
+// the exact sum of output (row i, column n) of an item from the operands in memory, rounded once and stored (the rare redo):
+// xo, co, oo: element offsets of X[j = 0], C[i, 0] and the output
+template <int L>
+__device__ __noinline__ void pm_exact(const PoleMmaArgs& a, i64 xo, i64 co, i64 oo, i64 E, i64 Er) {
+    constexpr int NW = 2 * L + 2;
+    const int jst = pm_jst(a);
+    u32 acc[NW];
+    zero(acc);
+    for (int j = 0; j < a.S; j++) {
+        u32 c[L], x[L], y[L];
+        const bool nc = load_mag<L>(a.cm, a.cplane, co + j, c), nx = load_mag<L>(a.xm, a.xplane, xo + (i64)j * jst, x);
+        const i64 ex = a.xe[xo + (i64)j * jst];
+        if (is_zero(c) || is_zero(x) || ex == EZ || E - ex >= 32 * L) continue;
+        shr(x, (int)(E - ex), y);
+        u32 prod[NW];                                               // schoolbook rows: a loop, not an unrolled product
+        zero(prod);
+#pragma unroll 1
+        for (int k = 0; k < L; k++) {
+            u64 cy = 0;
+#pragma unroll 1
+            for (int m = 0; m < L; m++) {
+                cy += (u64)c[k] * y[m] + prod[k + m];
+                prod[k + m] = (u32)cy;
+                cy >>= 32;
+            }
+            prod[k + L] = (u32)cy;
+        }
+        if (nc != nx) sub_borrow(acc, acc, prod, 0u);
+        else add_carry(acc, acc, prod, 0u);
+    }
+    store_rounded<L, NW>(a.om, a.oe, a.oplane, oo, acc, E + Er);
 }
 
-// Magnitude view of a two's complement limb column col[k * st] (k < NW): limb i of |value|.  With neg, z is
-// the lowest nonzero limb: -x = ~x + 1, and the +1 only reaches the limbs up to z.
-template <int NW>
-struct PmCol {
-    const u32* col;
-    int st, z, lo;                                                  // limbs below lo are zero
-    bool neg;
-    __device__ __forceinline__ u32 conv(int i, u32 v) const {
-        return neg ? (i > z ? ~v : (i == z ? 0u - v : 0u)) : v;
+// one column of a row: its positions d4 from P0 -> limbs (two's complement, one more for the sign)
+template <int L>
+__device__ __forceinline__ i64 pm_limbs(const int4* d4, u32 (&w)[PoleMmaGeom<L>::NPW + 1]) {
+    constexpr int NPW = PoleMmaGeom<L>::NPW;
+    i64 cy = 0;
+#pragma unroll
+    for (int q = 0; q < NPW; q++) {
+        const int4 d = d4[q];
+        const i64 x = (i64)d.x + (i64)d.y * 256 + ((i64)d.z + (i64)d.w * 256) * 65536;
+        const i64 s = x + cy;
+        w[q] = (u32)s;
+        cy = s >> 32;
     }
-    __device__ __forceinline__ u32 operator()(int i) const {
-        return (i < 0 || i >= NW) ? 0u : conv(i, col[i * st]);
-    }
-    __device__ __forceinline__ void init() {
-        neg = (col[(NW - 1) * st] >> 31) != 0;
-        z = lo;
-        if (neg)
-            while (z < NW - 1 && col[z * st] == 0) z++;
-    }
-    // bit length of the magnitude (0 for zero), by a scan from the top limb
-    __device__ __forceinline__ int bitlen() const {
-        for (int i = NW - 1; i >= lo; i--) {
-            const u32 m = (*this)(i);
-            if (m) return 32 * i + 32 - __clz(m);
-        }
-        return 0;
-    }
-};
+    w[NPW] = (u32)cy;
+    return cy;
+}
 
-// round_safe of mp.cuh on a magnitude view of bit length bl: every value within 2^(32 EW) rounds alike
-template <int L, int EW, class Mag>
-__device__ __forceinline__ bool pm_round_safe(const Mag& m, int bl) {
-    const int hb = bl - nb_bits(L) - 1;
-    if (hb < 32 * EW + 2) return false;
-    const u32 flip = ((m(hb >> 5) >> (hb & 31)) & 1u) ? 0u : ~0u;
-    for (int k = hb >> 5; k >= EW; k--) {
-        const int lo = 32 * k;
-        const u32 mask = hb >= lo + 32 ? ~0u : (hb > lo ? (1u << (hb - lo)) - 1u : 0u);
-        if ((m(k) ^ flip) & mask) return true;
+// sign, one rounding of a column's limbs, stored at output offset oo
+template <int L>
+__device__ __forceinline__ void pm_column(const PoleMmaArgs& a, u32 (&w)[PoleMmaGeom<L>::NPW + 1], i64 E, i64 Er, i64 xo, i64 co,
+                                          i64 oo) {
+    using G = PoleMmaGeom<L>;
+    constexpr int NB = nb_bits(L), NPW = G::NPW, NW = NPW + 1;
+    const bool neg = (w[NPW] >> 31) != 0;
+    if (neg) negate(w);
+    // bit length from the top limbs; the half bit of the rounding
+    int bl = 0;
+#pragma unroll
+    for (int k = NW - 4; k < NW; k++)
+        if (w[k]) bl = 32 * k + 32 - __clz(w[k]);
+    const int hb = bl - NB - 1, q = hb >> 5, f = hb & 31;
+    constexpr int Q0 = (32 * NPW - NB - 1) >> 5;                     // of a sum that fills its limbs; most lie in Q0 - 1, Q0
+    u32 r[L];
+    i64 er;
+    bool done = false;
+    if (Q0 >= 3 && bl != 0 && (q == Q0 || q == Q0 - 1)) {
+        u32 x[L + 3];                                               // limbs q - 1 .. q + L + 1
+#pragma unroll
+        for (int k = 0; k < L + 3; k++) {
+            const int hi = Q0 - 1 + k, lo = Q0 - 2 + k;
+            x[k] = q == Q0 ? (hi < NW ? w[hi < NW ? hi : 0] : 0u) : (lo >= 0 && lo < NW ? w[lo >= 0 && lo < NW ? lo : 0] : 0u);
+        }
+        const u32 below = fsr(x[0], x[1], f);                       // the 32 bits under the half bit (all above the error)
+        u32 t[L + 1];
+#pragma unroll
+        for (int k = 0; k <= L; k++) t[k] = fsr(x[k + 1], x[k + 2], f);
+        const u32 half = t[0] & 1u;
+        if (P0_exact<L>() || below != (half ? 0u : ~0u)) {          // no midpoint within the dropped part
+#pragma unroll
+            for (int k = 0; k < L; k++) r[k] = fsr(t[k], t[k + 1], 1);
+            add_bit(r, r, half);
+            int s = hb + 1;
+            if ((r[L - 1] >> (NB - 32 * (L - 1))) != 0) {            // rounded up to 2^NB
+#pragma unroll
+                for (int k = 0; k < L; k++) r[k] = fsr(r[k], k + 1 < L ? r[k + 1] : 0u, 1);
+                s++;
+            }
+            er = E + Er + 8 * G::P0 + s;
+            done = true;
+        }
+    } else if (P0_exact<L>() || round_safe<L, NW, 1>(w)) {           // other lengths: the general rounding
+        if (round_mag<L>(w, E + Er + 8 * G::P0, r, &er)) {
+            done = true;
+        } else {
+            zero(r);
+            er = EZ;
+            done = true;
+        }
+    }
+    if (!done) {
+        pm_exact<L>(a, xo, co, oo, E, Er);
+        return;
+    }
+    store_signed<L>(a.om, a.oplane, oo, r, neg && er != EZ);
+    a.oe[oo] = er;
+}
+
+// mbarrier wait, bounded, given up early once the CTA has failed
+__device__ __forceinline__ bool pm_wait(uint64_t* bar, uint32_t parity, const int* fail) {
+    const uint32_t addr = smem_u32(bar);
+    for (uint32_t it = 0; it < kWaitLimit; it++) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred P;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, P;\n\t}"
+            : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+        if (done) return true;
+        if ((it & 63) == 63 && *(const volatile int*)fail) return false;
     }
     return false;
 }
 
-// round_mag of mp.cuh on a magnitude view of bit length bl > 0: r and the exponent ein + shift, the same bits.
-// The L + 2 limbs the rounding reads are loaded in one batch from the run-time word offset.
-template <int L, int NW>
-__device__ __forceinline__ i64 pm_round(const PmCol<NW>& m, int bl, i64 ein, u32 (&r)[L]) {
-    constexpr int NB = nb_bits(L);
-    int s = bl - NB;
-    if (s <= 0) {                                                   // fewer than NB bits: exact left shift
-        const int q = (-s) >> 5, f = (-s) & 31;
-#pragma unroll
-        for (int k = 0; k < L; k++) r[k] = fsl(m(k - q - 1), m(k - q), f);
-        return ein + s;
-    }
-    const int q = (s - 1) >> 5, f = (s - 1) & 31;                  // q + L + 1 <= NW
-    u32 v[L + 2];
-#pragma unroll
-    for (int k = 0; k < L + 2; k++) v[k] = q + k < NW ? m.col[(q + k) * m.st] : 0u;
-#pragma unroll
-    for (int k = 0; k < L + 2; k++) v[k] = q + k < NW ? m.conv(q + k, v[k]) : 0u;
-    u32 t[L + 1];
-#pragma unroll
-    for (int k = 0; k <= L; k++) t[k] = fsr(v[k], v[k + 1], f);
-    u32 c = t[0] & 1u;
-#pragma unroll
-    for (int k = 0; k < L; k++) {
-        const u32 x = (t[k] >> 1) | (t[k + 1] << 31);
-        const u32 sum = x + c;
-        c = (c && sum == 0) ? 1u : 0u;
-        r[k] = sum;
-    }
-    if ((r[L - 1] >> (NB - 32 * (L - 1))) != 0) {
-#pragma unroll
-        for (int k = 0; k < L; k++) r[k] = (r[k] >> 1) | (k + 1 < L ? r[k + 1] << 31 : 0u);
-        s += 1;
-    }
-    return ein + s;
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// The rounding of one column decided by its header thread, so that every output limb can then be formed
-// on its own: magnitude limbs from the column (neg, z as in PmCol), x = floor(|sum| / 2^s) with s = 32 Q + F,
-// the half bit c0, the carry of the rounding reaching limbs 0 .. kc, and for the two's complement store the
-// lowest nonzero limb kz of the rounded magnitude.
-struct PmHead {
-    enum { kZero = 0, kLimbs = 1, kRenorm = 2, kDone = 3 };
-    int mode, s, Q, F, z, kc, kz, c0, neg;
-};
-
-template <int NW>
-__device__ __forceinline__ u32 pm_mag(const u32* col, int st, int i, bool neg, int z) {
-    if (i < 0 || i >= NW) return 0u;
-    const u32 v = col[i * st];
-    return neg ? (i > z ? ~v : (i == z ? 0u - v : 0u)) : v;
+// sixteen TMEM columns of a warp's lanes (not waited for)
+__device__ __forceinline__ void tmem_ld16(uint32_t* d, uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]),
+          "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
+        : "r"(addr));
 }
 
-template <int L, int NW>
-__device__ __forceinline__ PmHead pm_head(const PmCol<NW>& m, int bl) {
-    constexpr int NB = nb_bits(L);
-    PmHead h{};
-    h.s = bl - NB;
-    h.neg = m.neg;
-    h.z = m.z;
-    if (h.s <= 0) { h.mode = PmHead::kDone; return h; }
-    h.Q = h.s >> 5;
-    h.F = h.s & 31;
-    h.c0 = (int)((m((h.s - 1) >> 5) >> ((h.s - 1) & 31)) & 1u);
-    auto x = [&](int k) { return fsr(m(h.Q + k), m(h.Q + k + 1), h.F); };
-    h.mode = PmHead::kLimbs;
-    if (h.c0) {
-        int k = 0;
-        u32 xk = x(0);
-        while (xk == 0xFFFFFFFFu && k < L - 1) xk = x(++k);
-        h.kc = k;
-        h.kz = k;                                                   // rounded limbs below kc are zero, kc is not
-        if (k == L - 1 && xk + 1u == (1u << (NB - 32 * (L - 1)))) h.mode = PmHead::kRenorm;
-    } else {
-        h.kc = -1;
-        int k = 0;
-        while (k < L - 1 && x(k) == 0u) k++;
-        h.kz = k;
-    }
-    return h;
-}
+__device__ __forceinline__ void front_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-// limb k of the stored (two's complement) result of a header
-template <int L, int NW>
-__device__ __forceinline__ u32 pm_limb(const PmHead& h, const u32* col, int st, int k) {
-    constexpr int NB = nb_bits(L);
-    u32 r;
-    if (h.mode == PmHead::kZero) return 0u;
-    if (h.mode == PmHead::kRenorm) {
-        r = k == L - 1 ? 1u << (NB - 1 - 32 * (L - 1)) : 0u;
-        return h.neg ? (k == L - 1 ? 0u - r : (k < L - 1 ? 0u : ~r)) : r;
-    }
-    const u32 xk = fsr(pm_mag<NW>(col, st, h.Q + k, h.neg, h.z), pm_mag<NW>(col, st, h.Q + k + 1, h.neg, h.z), h.F);
-    r = xk + (k <= h.kc ? 1u : 0u);
-    if (!h.neg) return r;
-    return k < h.kz ? 0u : (k == h.kz ? 0u - r : ~r);
-}
-
-// limbs [w KQ, (w + 1) KQ) of the stored result (KQ = ceil(L / 4)), written to out[k * plane]: the KQ + 1
-// magnitude limbs they read are loaded once
-template <int L, int NW>
-__device__ __forceinline__ void pm_limbs(const PmHead& h, const u32* col, int st, int w, int32_t* out, i64 plane) {
-    constexpr int NB = nb_bits(L), KQ = (L + 3) / 4;
-    const int k0 = w * KQ;
-    if (h.mode != PmHead::kLimbs) {
-#pragma unroll
-        for (int q = 0; q < KQ; q++) {
-            const int k = k0 + q;
-            if (k < L) out[k * plane] = (int32_t)pm_limb<L, NW>(h, col, st, k);
-        }
-        return;
-    }
-    u32 mm[KQ + 1];
-#pragma unroll
-    for (int q = 0; q <= KQ; q++) mm[q] = pm_mag<NW>(col, st, h.Q + k0 + q, h.neg, h.z);
-#pragma unroll
-    for (int q = 0; q < KQ; q++) {
-        const int k = k0 + q;
-        if (k < L) {
-            const u32 r = fsr(mm[q], mm[q + 1], h.F) + (k <= h.kc ? 1u : 0u);
-            out[k * plane] = (int32_t)(!h.neg ? r : (k < h.kz ? 0u : (k == h.kz ? 0u - r : ~r)));
-        }
-    }
-    (void)NB;
-}
-
-// col (two's complement limbs, stride st) += sum_{p < P0} D[p, n] 256^p, from the digits in shared memory
-// (the rare exact redo)
-template <int L>
-__device__ void pm_add_low(u32* col, int st, const u32* cdig, const uint8_t* bop, int S, int NC, int n) {
-    using G = PoleMmaGeom<L>;
-    constexpr int P0 = G::P0, U = G::U, D = G::D;
-    i64 c = 0;
-    for (int k = 0; k < G::NW; k++) {
-        i64 v = 0;
-        if (k < P0 / 4) {
-            for (int r = 0; r < 4; r++) {
-                const int p = 4 * k + r;
-                i64 cp = 0;
-                for (int j = 0; j < S; j++) {
-                    const uint8_t* cd = reinterpret_cast<const uint8_t*>(cdig + j * G::CW) + G::PADB;
-                    for (int u = 0; u <= p && u < D; u++) {
-                        if (p - u >= D) continue;
-                        const int kap = j * U + (U - 1 - u);            // reversed digit index along K
-                        const int xd = sbyte(bop, (kap >> 4) * 16 * NC + (n >> 3) * 128 + (n & 7) * 16 + (kap & 15));
-                        cp += (i64)sbyte(cd, p - u) * xd;
-                    }
-                }
-                v += cp * ((i64)1 << (8 * r));
-            }
-        }
-        const i64 s = (i64)col[k * st] + v + c;
-        col[k * st] = (u32)s;
-        c = s >> 32;
-    }
+// barrier of the front warps; whether any of their threads passed true (the same answer for all)
+__device__ __forceinline__ bool front_any(bool x) {
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.s32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, 1, 128, p;\n\t"
+        "selp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(r) : "r"((int)x) : "memory");
+    return r != 0;
 }
 
 // warp 1, lane j < S: the digit string of c_ij (its magnitude and sign in c, ng) into a padded buffer
@@ -342,38 +296,44 @@ __device__ __forceinline__ void pm_put_digits(u32 (&c)[L], bool ng, u32* dst) {
 }
 
 template <int L>
-__global__ void __launch_bounds__(kPoleMmaThreads, 3) k_pole_mma(PoleMmaArgs a) {
+__global__ void __launch_bounds__(kPoleMmaThreads, 3) k_pole_mma(const __grid_constant__ PoleMmaArgs a) {
     using G = PoleMmaGeom<L>;
     using SM = PoleMmaSmem<L>;
-    constexpr int U = G::U, MT = G::MT, NW = G::NW, VW = G::VW, CW = G::CW, FAM = G::FAM, NWIN = G::NWIN,
-                  DS = G::DS, P0 = G::P0;
+    constexpr int U = G::U, NCH = G::NCH, MT = G::MT, CW = G::CW, FAM = G::FAM, NWIN = G::NWIN, DS = G::DS, NP = G::NP;
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bar, dfull, dempty;             // MMAs of a row; slot filled, slot read out
     __shared__ uint32_t tmem_sh;
     __shared__ int fail_sh;
-    __shared__ i64 carr[8][kPoleMmaMaxNC];                          // carry out of each chain segment
     __shared__ i64 er_sh[kPoleMmaMaxS];                             // row exponents of the task's constant
-    __shared__ PmHead head[kPoleMmaMaxNC];                          // the rounding of each column
     __shared__ int coff_sh[kPoleMmaMaxNC];                          // column offsets inside the task's block
 
     const int S = a.S, NC = a.NC, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ncs = NC == 32 ? 5 : 4;                               // NC is 16 or 32
-    const bool cthread = warp == 1 && lane < S;                     // the constants' digit strings
     const i64 N = (i64)S * a.B;
     uint8_t* bop = smem;
     uint8_t* hank = smem + SM::bop(S, NC);
-    u32* dbuf = reinterpret_cast<u32*>(hank);                       // D[n][p]: reuses the windows after the MMAs
-    u32* accs = dbuf + (size_t)NC * DS;                              // limb k of column n at accs[k * (NC + 1) + n]
-    const int ast = NC + 1;
-    u32* cdig = reinterpret_cast<u32*>(hank + SM::hank(S, NC));    // row r at cdig + (r % 2) S CW
-    i64* ecol = reinterpret_cast<i64*>(reinterpret_cast<uint8_t*>(cdig) + SM::cdig(S));
+    u32* cdig = reinterpret_cast<u32*>(hank + SM::hank(S));         // row r at cdig + (r % 2) S CW
+    u32* dbuf = cdig + SM::cdig(S) / 4;                             // D[n][p]
+    i64* ecol = reinterpret_cast<i64*>(reinterpret_cast<uint8_t*>(dbuf) + SM::slot(NC));   // the item's column exponents
+    i64* inf = ecol + kPoleMmaMaxNC + 1;                            // the slot's, and its row's
+    uint64_t* adesc = reinterpret_cast<uint64_t*>(inf + kPoleMmaMaxNC + 1);   // A descriptor of each K step
+    const int nsteps = SM::steps(S);
     uint32_t ncols = 32;
     while (ncols < (uint32_t)(MT * NC)) ncols <<= 1;
 
     for (int q = tid; q < 2 * S * CW; q += blockDim.x) cdig[q] = 0;   // padding stays zero: digits go to [PADB, PADB + D)
+    // K step s multiplies chunks 2 s and 2 s + 1 of the row of entries (entry g / NCH, 16 windows on per chunk)
+    for (int q = tid; q < nsteps; q += blockDim.x) {
+        auto at = [&](int g) { return (g / NCH) * FAM + (g % NCH) * 256; };
+        const int g = 2 * q;
+        adesc[q] = umma_desc(smem_u32(hank) + at(g), g + 1 < S * NCH ? at(g + 1) - at(g) : 256, 128);
+    }
+    for (int q = tid; q < NC; q += blockDim.x)                       // the chunk after the last entry: zero
+        if ((S * NCH) & 1) *reinterpret_cast<uint4*>(bop + (size_t)S * NCH * 16 * NC + 16 * q) = make_uint4(0, 0, 0, 0);
     if (tid == 0) {
         fail_sh = 0;
         mbar_init(&bar, 1);
+        mbar_init(&dfull, 128);
+        mbar_init(&dempty, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -385,278 +345,208 @@ __global__ void __launch_bounds__(kPoleMmaThreads, 3) k_pole_mma(PoleMmaArgs a) 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_sh;
-    // instruction descriptor: s32 accumulator, s8 x s8, both K-major, M = 128, N = NC
-    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    // descriptors of the first A and B core matrices; the others differ only in the 14-bit address field
-    const uint64_t da0 = umma_desc(smem_u32(hank), 256, 128), db0 = umma_desc(smem_u32(bop), 16 * NC, 128);
-    uint32_t phase = 0;
-    int pending = 0;                                                // thread 0: a commit not yet waited for
-
     const i64 items = a.T * a.nchunks;
-    for (i64 w = blockIdx.x; w < items; w += gridDim.x) {
-        const i64 t = w / a.nchunks;
-        const i64 n0 = (w % a.nchunks) * (i64)NC;
-        const int nn = (int)(N - n0 < NC ? N - n0 : NC);
-        const i64 xrow = a.t_x ? a.t_x[t] : t, crow = a.t_c[t], orow = a.t_o ? a.t_o[t] : t;
+    const int jst = pm_jst(a);
+    bool pending = false;                                           // thread 0: a commit not yet waited for
+    uint32_t phase = 0;
 
-        // 1. the constants of row 0 (digits now) and row 1 (loaded, converted during row 0), row exponents
-        u32 cn[L];
-        bool cneg = false;
-        if (cthread) {
-            cneg = load_mag<L>(a.cm, a.cplane, crow * S * S + lane, cn);
-            er_sh[lane] = a.ce[crow * S + lane];
-            pm_put_digits<L>(cn, cneg, cdig + lane * CW + G::PADB / 4);
-            if (S > 1) cneg = load_mag<L>(a.cm, a.cplane, (crow * S + 1) * S + lane, cn);
-        }
-        const i64 xbase = xrow * S * S * a.B, obase = orow * S * S * a.B;
-        const int jst = pm_jst(a);
-        // column exponents: the largest over j of the nonzero entries (all loads of a column issued at once)
-        for (int n = tid; n < NC; n += blockDim.x) {
-            i64 E = EZ;
-            const int co = n < nn ? pm_coff(a, (int)n0 + n) : 0;
-            coff_sh[n] = co;
-            if (n < nn) {
-                i64 ev[kPoleMmaMaxS];
-                int32_t tv[kPoleMmaMaxS];
+    if (warp == 4) {                                                // back warp
+        u32 row = 0;
+        bool stop = false;
+        for (i64 w = blockIdx.x; w < items && !stop; w += gridDim.x) {
+            const i64 t = w / a.nchunks, n0 = (w % a.nchunks) * (i64)NC;
+            const int nn = (int)(N - n0 < NC ? N - n0 : NC);
+            const i64 xrow = a.t_x ? a.t_x[t] : t, crow = a.t_c[t], orow = a.t_o ? a.t_o[t] : t;
+            const i64 xbase = xrow * S * S * a.B, obase = orow * S * S * a.B;
+            const int co = lane < nn ? pm_coff(a, (int)n0 + lane) : 0;
+            for (int i = 0; i < S; i++, row++) {
+                if (!__all_sync(0xFFFFFFFFu, pm_wait(&dfull, row & 1u, &fail_sh))) {
+                    if (lane == 0) atomicCAS(&fail_sh, 0, 3);
+                    stop = true;
+                    break;
+                }
+                const i64 E = inf[lane & (NC - 1)], Er = inf[kPoleMmaMaxNC], oo = obase + co + (i64)i * jst;
+                u32 wd[G::NPW + 1];
+                pm_limbs<L>(reinterpret_cast<const int4*>(dbuf + (lane & (NC - 1)) * DS), wd);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&dempty);
+                if (lane < nn) {
+                    if (E == EZ || Er == EZ) {
 #pragma unroll
-                for (int j = 0; j < kPoleMmaMaxS; j++) {
-                    if (j < S) {
-                        const i64 ix = xbase + co + j * jst;
-                        ev[j] = a.xe[ix];
-                        tv[j] = a.xm[(L - 1) * a.xplane + ix];
+                        for (int k = 0; k < L; k++) a.om[k * a.oplane + oo] = 0;
+                        a.oe[oo] = EZ;
+                    } else {
+                        pm_column<L>(a, wd, E, Er, xbase + co, (crow * S + i) * S, oo);
                     }
                 }
-#pragma unroll
-                for (int j = 0; j < kPoleMmaMaxS; j++)
-                    if (j < S && tv[j] != 0 && ev[j] > E) E = ev[j];
-            }
-            ecol[n] = E;
-        }
-        __syncthreads();
-        // the aligned X digits into the B operand
-        for (int it = tid; it < S * NC; it += blockDim.x) {
-            const int j = it >> ncs, n = it & (NC - 1);
-            u32 dg[L];
-            zero(dg);
-            const i64 E = ecol[n];
-            if (n < nn) {
-                const i64 ix = xbase + coff_sh[n] + j * jst;
-                u32 x[L];
-                const bool neg = load_mag<L>(a.xm, a.xplane, ix, x);
-                const i64 ex = a.xe[ix];
-                if (E != EZ && !is_zero(x) && ex != EZ && E - ex < 32 * L) {
-                    shr(x, (int)(E - ex), dg);
-                    if (neg) negate(dg);
-                }
-            }
-            to_balanced(dg);
-            uint8_t* col = bop + (n >> 3) * 128 + (n & 7) * 16;
-#pragma unroll
-            for (int c = 0; c < U / 16; c++) {
-                u32 q[4];
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const int wd = U / 4 - 1 - (4 * c + r);            // reversed words, bytes reversed inside
-                    q[r] = wd < L ? __byte_perm(dg[wd], 0, 0x0123) : 0u;
-                }
-                *reinterpret_cast<uint4*>(col + (size_t)(j * (U / 16) + c) * 16 * NC) = make_uint4(q[0], q[1], q[2], q[3]);
             }
         }
-        __syncthreads();
-
-        // 2. rows
+    } else {
+        const int ncs = NC == 32 ? 5 : 4;                           // NC is 16 or 32
+        const bool cthread = warp == 1 && lane < S;                 // the constants' digit strings
+        // instruction descriptor: s32 accumulator, s8 x s8, both K-major, M = 128, N = NC
+        const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        // B descriptor of the first K step; the others differ only in the 14-bit address field
+        const uint64_t db0 = umma_desc(smem_u32(bop), 16 * NC, 128);
+        u32 row = 0;
         bool stop = false;
-        for (int i = 0; i < S; i++) {
-            const i64 Er = er_sh[i];
-            const u32* cd = cdig + (i & 1) * S * CW;
-            if (Er == EZ) {                                          // a zero row of the constant: exact zeros
-                for (int n = tid; n < nn; n += blockDim.x) pm_store_zero<L>(a, obase + coff_sh[n] + i * jst);
-                if (cthread && i + 1 < S) {
-                    pm_put_digits<L>(cn, cneg, cdig + ((i + 1) & 1) * S * CW + lane * CW + G::PADB / 4);
-                    if (i + 2 < S) cneg = load_mag<L>(a.cm, a.cplane, (crow * S + i + 2) * S + lane, cn);
-                }
-                __syncthreads();
-                continue;
+        for (i64 w = blockIdx.x; w < items && !stop; w += gridDim.x) {
+            const i64 t = w / a.nchunks, n0 = (w % a.nchunks) * (i64)NC;
+            const int nn = (int)(N - n0 < NC ? N - n0 : NC);
+            const i64 xrow = a.t_x ? a.t_x[t] : t, crow_now = a.t_c[t];
+
+            // the constants of row 0 (digits now) and row 1 (loaded, converted during row 0), row exponents
+            u32 cn[L];
+            bool cneg = false;
+            if (cthread) {
+                cneg = load_mag<L>(a.cm, a.cplane, crow_now * S * S + lane, cn);
+                er_sh[lane] = a.ce[crow_now * S + lane];
+                pm_put_digits<L>(cn, cneg, cdig + lane * CW + G::PADB / 4);
+                if (S > 1) cneg = load_mag<L>(a.cm, a.cplane, (crow_now * S + 1) * S + lane, cn);
             }
-            // windows o .. o + 3 (o a multiple of 4) start at bytes P0 + 1 + o .. of the padded string: words
-            // ws .. ws + 4 shifted by 1 to 4 bytes.  The thread stores them in the rotated order k' = (k + t / 2) % 4
-            // so that the eight threads of each store phase cover all 32 banks.
-            for (int it = tid; it < S * (NWIN / 4); it += blockDim.x) {
-                const int j = it / (NWIN / 4), o = 4 * (it % (NWIN / 4));
-                const u32* cw = cd + j * CW + ((P0 + o) >> 2);
-                const u32 w0 = cw[0], w1 = cw[1], w2 = cw[2], w3 = cw[3], w4 = cw[4];
-                uint4* dst = reinterpret_cast<uint4*>(hank + (size_t)j * FAM + 16 * o);
+            const i64 xbase = xrow * S * S * a.B;
+            // column exponents: the largest over j of the nonzero entries (all loads of a column issued at once)
+            i64 Ec = EZ;
+            if (tid < NC) {
+                const int n = tid, co = n < nn ? pm_coff(a, (int)n0 + n) : 0;
+                coff_sh[n] = co;
+                if (n < nn) {
+                    i64 ev[kPoleMmaMaxS];
+                    int32_t tv[kPoleMmaMaxS];
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int kp = (k + (tid >> 1)) & 3;
-                    const u32 sel = 0x4321u + 0x1111u * (u32)kp;
-                    dst[kp] = make_uint4(__byte_perm(w0, w1, sel), __byte_perm(w1, w2, sel), __byte_perm(w2, w3, sel),
-                                         __byte_perm(w3, w4, sel));
+                    for (int j = 0; j < kPoleMmaMaxS; j++) {
+                        if (j < S) {
+                            const i64 ix = xbase + co + j * jst;
+                            ev[j] = a.xe[ix];
+                            tv[j] = a.xm[(L - 1) * a.xplane + ix];
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kPoleMmaMaxS; j++)
+                        if (j < S && tv[j] != 0 && ev[j] > Ec) Ec = ev[j];
+                }
+                ecol[n] = Ec;
+            }
+            front_sync();
+            // the aligned X digits into the B operand
+            for (int it = tid; it < S * NC; it += 128) {
+                const int j = it >> ncs, n = it & (NC - 1);
+                u32 dg[L];
+                zero(dg);
+                const i64 E = ecol[n];
+                if (n < nn) {
+                    const i64 ix = xbase + coff_sh[n] + j * jst;
+                    u32 x[L];
+                    const bool neg = load_mag<L>(a.xm, a.xplane, ix, x);
+                    const i64 ex = a.xe[ix];
+                    if (E != EZ && !is_zero(x) && ex != EZ && E - ex < 32 * L) {
+                        shr(x, (int)(E - ex), dg);
+                        if (neg) negate(dg);
+                    }
+                }
+                to_balanced(dg);
+                uint8_t* col = bop + (n >> 3) * 128 + (n & 7) * 16;
+#pragma unroll
+                for (int c = 0; c < U / 16; c++) {
+                    u32 q[4];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const int wd = U / 4 - 1 - (4 * c + r);        // reversed words, bytes reversed inside
+                        q[r] = wd < L ? __byte_perm(dg[wd], 0, 0x0123) : 0u;
+                    }
+                    *reinterpret_cast<uint4*>(col + (size_t)(j * (U / 16) + c) * 16 * NC) = make_uint4(q[0], q[1], q[2], q[3]);
                 }
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> tensor-core reads
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncthreads();
-            if (tid == 0) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-                for (int mt = 0; mt < MT; mt++) {
-#pragma unroll 1
-                    for (int j = 0; j < S; j++) {
-                        const uint64_t da = da0 + (uint64_t)((j * FAM + 2048 * mt) >> 4);
-                        const uint64_t db = db0 + (uint64_t)((j * (U / 16) * 16 * NC) >> 4);
+            for (int i = 0; i < S; i++, row++) {
+                const i64 Er = er_sh[i];
+                const u32* cd = cdig + (i & 1) * S * CW;
+                if (Er != EZ) {
+                    // windows o .. o + 3 (o a multiple of 4) start at bytes 1 + o .. of the padded string: words
+                    // o / 4 .. o / 4 + 4 shifted by 1 to 4 bytes.  The thread stores them in the rotated order
+                    // k' = (k + t / 2) % 4 so that the eight threads of each store phase cover all 32 banks.
+                    for (int it = tid; it < S * (NWIN / 4); it += 128) {
+                        const int j = it / (NWIN / 4), o = 4 * (it % (NWIN / 4));
+                        const u32* cw = cd + j * CW + (o >> 2);
+                        const u32 w0 = cw[0], w1 = cw[1], w2 = cw[2], w3 = cw[3], w4 = cw[4];
+                        uint4* dst = reinterpret_cast<uint4*>(hank + (size_t)j * FAM + 16 * o);
 #pragma unroll
-                        for (int ks = 0; ks < U / 32; ks++) {
-                            const uint32_t accf = (j > 0 || ks > 0) ? 1u : 0u;
+                        for (int k = 0; k < 4; k++) {
+                            const int kp = (k + (tid >> 1)) & 3;
+                            const u32 sel = 0x4321u + 0x1111u * (u32)kp;
+                            dst[kp] = make_uint4(__byte_perm(w0, w1, sel), __byte_perm(w1, w2, sel), __byte_perm(w2, w3, sel),
+                                                 __byte_perm(w3, w4, sel));
+                        }
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> tensor-core reads
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                front_sync();
+                if (tid == 0 && Er != EZ) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int mt = 0; mt < MT; mt++) {
+#pragma unroll 4
+                        for (int ks = 0; ks < nsteps; ks++) {
+                            const uint32_t accf = ks > 0 ? 1u : 0u;
                             asm volatile(
                                 "{\n\t.reg .pred p;\n\t"
                                 "setp.ne.b32 p, %4, 0;\n\t"
                                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                                ::"r"(tmem + (uint32_t)(mt * NC)), "l"(da + (uint64_t)(32 * ks)),
-                                  "l"(db + (uint64_t)(2 * ks * NC)), "r"(idesc), "r"(accf) : "memory");
+                                ::"r"(tmem + (uint32_t)(mt * NC)), "l"(adesc[ks] + (uint64_t)(128 * mt)),
+                                  "l"(db0 + (uint64_t)(2 * ks * NC)), "r"(idesc), "r"(accf) : "memory");
                         }
                     }
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                                 ::"r"(smem_u32(&bar)) : "memory");
+                    pending = true;
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                             ::"r"(smem_u32(&bar)) : "memory");
-                pending = 1;
-                if (!mbar_wait(&bar, phase, kWaitLimit)) fail_sh = 1;
-                else pending = 0;
-            } else if (cthread && i + 1 < S) {                       // next row's digits while the MMAs run
-                pm_put_digits<L>(cn, cneg, cdig + ((i + 1) & 1) * S * CW + lane * CW + G::PADB / 4);
-                if (i + 2 < S) cneg = load_mag<L>(a.cm, a.cplane, (crow * S + i + 2) * S + lane, cn);
-            }
-            phase ^= 1;
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncthreads();
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (fail_sh) { stop = true; break; }
-
-            // 3. per tile of 128 positions: accumulators -> D[n][p] in shared memory (this lane's position p,
-            // sixteen columns per load), then the carry chain in four segments of eight limbs (warp s: words
-            // 32 mt + 8 s .. + 8 of every column, lane = column), each from a zero carry; the carries out are
-            // joined below
+                if (cthread && i + 1 < S) {                          // next row's digits while the MMAs run
+                    pm_put_digits<L>(cn, cneg, cdig + ((i + 1) & 1) * S * CW + lane * CW + G::PADB / 4);
+                    if (i + 2 < S) cneg = load_mag<L>(a.cm, a.cplane, (crow_now * S + i + 2) * S + lane, cn);
+                }
+                bool bad = false;
+                if (Er != EZ) {
+                    bad = !pm_wait(&bar, phase, &fail_sh);
+                    if (bad) atomicCAS(&fail_sh, 0, 1);
+                    else pending = false;
+                    phase ^= 1;
+                }
+                if (!bad && row > 0 && !pm_wait(&dempty, (row - 1) & 1u, &fail_sh)) {
+                    bad = true;
+                    atomicCAS(&fail_sh, 0, 4);
+                }
+                if (front_any(bad)) { stop = true; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                // accumulators -> D[n][p] of the slot (this lane's position p)
+                if (Er != EZ) {
 #pragma unroll 1
-            for (int mt = 0; mt < MT; mt++) {
-                const int p = warp * 32 + lane;
+                    for (int mt = 0; mt < MT; mt++) {
+                        if (mt * 128 + warp * 32 >= NP) break;
+                        const int p = mt * 128 + warp * 32 + lane;
 #pragma unroll 1
-                for (int c0 = 0; c0 < NC; c0 += 16) {
-                    uint32_t d[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]),
-                          "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]),
-                          "=r"(d[14]), "=r"(d[15])
-                        : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * NC + c0)));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        for (int c0 = 0; c0 < NC; c0 += 16) {
+                            uint32_t d[16];
+                            tmem_ld16(d, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * NC + c0));
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                            if (p < NP) {
 #pragma unroll
-                    for (int q = 0; q < 16; q++) dbuf[(c0 + q) * DS + p] = d[q];
-                }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncthreads();
-                if (lane < nn) {
-                    const int n = lane;
-                    u32* col = accs + n;
-                    const int4* dn = reinterpret_cast<const int4*>(dbuf + (size_t)n * DS);
-                    i64 c = 0;
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const int k = P0 / 4 + 32 * mt + 8 * warp + q;
-                        if (k < NW) {
-                            const int4 d = dn[8 * warp + q];
-                            const i64 s = c + (i64)d.x + (i64)d.y * 256 + (i64)d.z * 65536 + (i64)d.w * 16777216;
-                            col[k * ast] = (u32)s;
-                            c = s >> 32;
-                        }
-                    }
-                    carr[4 * mt + warp][n] = c;
-                }
-                __syncthreads();
-            }
-
-            // join the segments, check the rounding (exact redo of the low positions where needed) and decide the
-            // rounded number: one header thread per column (column n on warp n % 4, lane n / 4)
-            {
-                const int n = 4 * lane + warp;
-                if (n < nn) {
-                    PmHead h{};
-                    h.mode = PmHead::kZero;
-                    const i64 out = obase + coff_sh[n] + i * jst;
-                    const i64 E = ecol[n];
-                    if (E != EZ) {
-                        u32* col = accs + n;
-                        // segment sg (sg >= 1) receives the carry out of segment sg - 1 (all segments at once);
-                        // what then runs out of the top of a segment (rare) is passed on in order afterwards
-                        constexpr int NSEG = 4 * MT;
-                        i64 e[NSEG];
-#pragma unroll
-                        for (int sg = 0; sg < NSEG; sg++) {
-                            i64 c = sg > 0 ? carr[sg - 1][n] : 0;
-                            const int k0 = P0 / 4 + 8 * sg, kend = k0 + 8 < NW ? k0 + 8 : NW;
-                            for (int k = k0; c != 0 && k < kend; k++) {
-                                const i64 v = (i64)col[k * ast] + c;
-                                col[k * ast] = (u32)v;
-                                c = v >> 32;
-                            }
-                            e[sg] = c;
-                        }
-                        i64 x = 0;
-#pragma unroll
-                        for (int sg = 1; sg < NSEG; sg++) {
-                            x += e[sg - 1];
-                            const int k0 = P0 / 4 + 8 * sg, kend = k0 + 8 < NW ? k0 + 8 : NW;
-                            for (int k = k0; x != 0 && k < kend; k++) {
-                                const i64 v = (i64)col[k * ast] + x;
-                                col[k * ast] = (u32)v;
-                                x = v >> 32;
+                                for (int q = 0; q < 16; q++) dbuf[(c0 + q) * DS + p] = d[q];
                             }
                         }
-                        i64 C = carr[NSEG - 1][n] + x + e[NSEG - 1];
-                        for (int k = P0 / 4 + VW; k < NW; k++) {
-                            col[k * ast] = (u32)C;
-                            C >>= 32;
-                        }
-                        PmCol<NW> m{col, ast, 0, P0 / 4, false};
-                        m.init();
-                        int bl = m.bitlen();
-                        if (P0 > 0 && !pm_round_safe<L, G::EW>(m, bl)) {
-                            for (int k = 0; k < P0 / 4; k++) col[k * ast] = 0u;
-                            pm_add_low<L>(col, ast, cd, bop, S, NC, n);
-                            m.lo = 0;
-                            m.init();
-                            bl = m.bitlen();
-                        }
-                        if (bl > 0) h = pm_head<L, NW>(m, bl);
-                        if (h.mode == PmHead::kDone) {                   // fewer than NB bits: rounded here
-                            u32 r[L];
-                            const i64 er = pm_round<L, NW>(m, bl, E + Er, r);
-                            store_signed<L>(a.om, a.oplane, out, r, m.neg);
-                            a.oe[out] = er;
-                        } else if (h.mode != PmHead::kZero) {
-                            a.oe[out] = E + Er + h.s + (h.mode == PmHead::kRenorm ? 1 : 0);
-                        }
                     }
-                    if (h.mode == PmHead::kZero) a.oe[out] = EZ;
-                    head[n] = h;
                 }
+                if (tid < NC) inf[tid] = Ec;
+                if (tid == 0) inf[kPoleMmaMaxNC] = Er;
+                mbar_arrive(&dfull);
             }
-            __syncthreads();
-            // the rounded limbs: a quarter of the limbs per warp, a lane per column, so that each limb plane is
-            // written in runs of consecutive outputs
-            if (lane < nn) {
-                const PmHead h = head[lane];
-                const i64 out = obase + coff_sh[lane] + i * jst;
-                if (h.mode != PmHead::kDone) pm_limbs<L, NW>(h, accs + lane, ast, warp, a.om + out, a.oplane);
-            }
-            __syncthreads();                                         // D, the limb columns and windows are reused
         }
-        if (stop) break;
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    __syncthreads();
     if (tid == 0 && pending) {                                       // bounded drain of our own MMAs
         if (!mbar_wait(&bar, phase ^ 1, kWaitLimit)) fail_sh = 2;
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
@@ -665,7 +555,9 @@ __global__ void __launch_bounds__(kPoleMmaThreads, 3) k_pole_mma(PoleMmaArgs a) 
 }
 
 #ifdef B3D_DEFINE_LAUNCH
-// columns per work item: all of a task's S B columns up to kPoleMmaMaxNC, in multiples of 16 (the MMA's N step)
+// columns per work item: all of a task's S B columns up to kPoleMmaMaxNC, in multiples of 16 (the MMA's N step).  64 columns
+// (the MMAs are bound by their A operand: a second 32 cost little) measured 0.84 to 1.0 of the time at S = 3 and 1.0 to 1.6
+// at S = 4, 5, where fewer CTAs fit.
 inline int pole_mma_nc(i64 N) { return (int)(N >= kPoleMmaMaxNC ? kPoleMmaMaxNC : ((N + 15) / 16) * 16); }
 
 template <int L>
@@ -675,7 +567,7 @@ static int pole_mma_stage(PoleMmaArgs a, cudaStream_t st) {
     static unsigned long long configured = 0;                       // devices whose limits are raised
     const unsigned long long dbit = device_bit();
     if (!(configured & dbit) || !dbit) {
-        int rc = (int)cudaFuncSetAttribute(k_pole_mma<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        int rc = (int)cudaFuncSetAttribute(k_pole_mma<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
         if (!rc) rc = (int)cudaFuncSetAttribute(k_pole_mma<L>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         if (rc) return rc;
         configured |= dbit;
@@ -684,8 +576,8 @@ static int pole_mma_stage(PoleMmaArgs a, cudaStream_t st) {
     int rc = (int)cudaGetDevice(&dev);
     if (!rc) rc = (int)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (rc) return rc;
-    // resident CTAs per SM: three by the launch bounds (registers), fewer when the shared memory (228 KB per
-    // SM: static + dynamic + 1 KB reserved per CTA) or the 512 TMEM columns do not hold three
+    // resident CTAs per SM: three by the launch bounds (registers), fewer when the shared memory (228 KB per SM: static +
+    // dynamic + 1 KB reserved per CTA) or the 512 TMEM columns do not hold three
     static size_t static_smem = 0;
     if (!static_smem) {
         cudaFuncAttributes fa;

@@ -24,22 +24,34 @@ CAUCHY = "cuda5"
 POLE = "auto"
 # Which pole-step form is faster.  The tensor-core form takes a task's S B columns in chunks of 32 at a cost per
 # chunk that hardly depends on how many columns are in use; the CUDA-core form costs in proportion to the
-# columns.  Measured on a B200 (both forms, both stages, 3000 synthetic tasks per shape, L in {26, 30, 34, 42},
-# S in {2 .. 5}, S B from 5 to 130): the time ratio CUDA cores / tensor cores of a full chunk, by (L, S); for other
-# column counts the ratio scales with the chunks' fill (S B / (32 chunks)) to within a few percent.
+# columns.  Measured on a B200 (both forms, both stages, 3000 synthetic tasks per shape, S in {2 .. 5}, S B from 5 to 252):
+# the time ratio CUDA cores / tensor cores of a full chunk, by (L, S); for other column counts the ratio scales with
+# the chunks' fill (S B / (32 chunks)) to within some percent on the low side (half a chunk: 0.96 measured for 0.86).
+POLE_SPEEDUP = {10: (0.67, 0.85, 1.02, 1.11), 18: (0.89, 1.17, 1.44, 1.56), 26: (1.12, 1.45, 1.75, 1.90),
+                30: (1.03, 1.35, 1.57, 1.62), 34: (1.13, 1.45, 1.67, 1.73), 42: (1.25, 1.54, 1.83, 1.37)}   # S = 2, 3, 4, 5
+# The same of the tensor-core kernel that took a row in four warps by turns, pole_mma_gain's model.
 POLE_FULL_CHUNK_RATIO = {26: (0.71, 0.91, 1.09, 1.23), 30: (0.64, 0.85, 1.02, 1.14), 34: (0.73, 0.93, 1.09, 1.24),
                          42: (0.90, 1.15, 1.32, 1.51)}            # S = 2, 3, 4, 5
 POLE_MIN_GAIN = 1.05
 
 
-def pole_mma_gain(L, S, B):
-    """predicted time ratio CUDA-core / tensor-core pole step (above 1: the tensor cores are faster)"""
+def _chunk_ratio(table, L, S, B):
     if S < 2:
         return 0.0
-    Lk = max((k for k in POLE_FULL_CHUNK_RATIO if k <= L), default=26)
-    r = POLE_FULL_CHUNK_RATIO[Lk][min(S, 5) - 2]
+    Lk = max((k for k in table if k <= L), default=min(table))
     cols = S * B
-    return r * cols / (32 * -(-cols // 32))
+    return table[Lk][min(S, 5) - 2] * cols / (32 * -(-cols // 32))
+
+
+def pole_mma_speedup(L, S, B):
+    """predicted time ratio CUDA-core / tensor-core pole step (above 1: the tensor cores are faster)"""
+    return _chunk_ratio(POLE_SPEEDUP, L, S, B)
+
+
+def pole_mma_gain(L, S, B):
+    """the ratio by the model of the earlier tensor-core kernel (POLE_FULL_CHUNK_RATIO); the choice of a run goes by
+    pole_mma_speedup"""
+    return _chunk_ratio(POLE_FULL_CHUNK_RATIO, L, S, B)
 
 
 def cauchy_fp_size(L, dmax, nb, Kc, N):
@@ -66,7 +78,7 @@ class Recursion:
         (the level's Cauchy GEMM on the tensor cores, residues + CRT), or "auto" (rns for levels with at least
         rns_min_k columns, cuda2 below).  pole: "mma" (the pole step's exact sums on the INT8 tensor cores,
         b3d_pole_level_mma; plans with Smax <= 8), "cuda" (b3d_pole_level) or "auto" (mma where the measured
-        crossover, pole_mma_gain, predicts it faster, cuda elsewhere): bit-identical"""
+        crossover, pole_mma_speedup, predicts it faster, cuda elsewhere): bit-identical"""
         self.cauchy, self.rns_min_k = cauchy or CAUCHY, rns_min_k
         self.pole = pole or POLE
         if self.pole not in ("mma", "cuda", "auto"):
@@ -292,7 +304,7 @@ class Recursion:
         """whether run() with B right-hand sides takes the tensor-core pole step"""
         if self.pole != "auto":
             return self.pole == "mma"
-        return pole_mma_gain(self.L, self.plan.Smax, B) >= POLE_MIN_GAIN
+        return pole_mma_speedup(self.L, self.plan.Smax, B) >= POLE_MIN_GAIN
 
     def check_errors(self):
         """raise B3DError if a kernel of this recursion gave up a bounded wait (synchronises the device)"""

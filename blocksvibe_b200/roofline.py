@@ -31,7 +31,8 @@ def pole_level_macs(lev, N, S):
 
 
 def pole_mma_geometry(L):
-    """(U, MT): digits per entry along K and 128-position tiles of the tensor-core pole step (pole_mma.cuh)"""
+    """(U, MT): digits per entry along K, padded to whole K steps, and 128-position tiles of the tensor-core pole step
+    (pole_mma.cuh, which packs the entries in chunks of 16 digits: up to 10 % fewer steps than U counts)"""
     NB, D = 32 * L - 2, 4 * L
     U = 32 * (-(-D // 32))
 
