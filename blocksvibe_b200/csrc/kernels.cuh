@@ -123,45 +123,9 @@ __global__ void __launch_bounds__(kAlignThreads) k_align_r(const int32_t* __rest
         align_one<L>(m, e, plane, base + k * sk, E, om, oplane, kmajor ? (b * K + k) * R + r : t * K + k);
 }
 
-// Exact sums of products, rounded once, computed in two tries (the pole steps).  The first drops the product columns below
-// trunc_cols<L>() (mac_signed_mem), which leaves the accumulator within 2^(32 (trunc_cols + 2)) of the exact sum;
-// where round_safe shows that no value that close rounds differently, its rounding is the exact sum's.  Elsewhere
-// (heavy cancellation, a sum at a rounding midpoint, exact zeros) the second try redoes the sum exactly.  With
-// both operands normalised a product has about 64 L bits and the rounding bit sits near bit 32 L, so the first
-// try has some 90 bits to spare.
+// The pole steps first drop the product columns below trunc_cols<L>() (mac_signed_win).  With both operands normalised a
+// product has about 64 L bits and the rounding bit sits near bit 32 L, so this leaves some 90 bits to spare.
 template <int L> B3D_CX int trunc_cols() { return L >= 10 ? L - 5 : 0; }
-
-// sum(std::integral_constant<int, C0>) fills the two's complement accumulator (limb w at acc[w * stride]) and
-// returns whether it added any product.  mag receives the magnitude of an accumulator whose rounding equals the
-// exact sum's; the return value is its sign.
-template <int L, int NW, class Sum> __device__ __forceinline__ bool exact_sum(Sum& sum, u32* acc, int stride,
-                                                                               u32 (&mag)[NW]) {
-    constexpr int C0 = trunc_cols<L>();
-    auto load = [&]() {
-#pragma unroll
-        for (int w = 0; w < NW; w++) mag[w] = acc[w * stride];
-        const bool neg = (mag[NW - 1] >> 31) != 0;
-        if (neg) negate(mag);
-        return neg;
-    };
-    const bool any = sum(std::integral_constant<int, C0>());
-    bool neg = load();
-    if (C0 > 0 && any && !round_safe<L, NW, C0 + 2>(mag)) {
-        sum(std::integral_constant<int, 0>());
-        neg = load();
-    }
-    return neg;
-}
-
-// Round a magnitude (NW limbs, value mag * 2^ein) and store it normalised with the given sign.
-template <int L, int NW> __device__ __forceinline__ void store_rounded_mag(int32_t* m, i64* e, i64 plane, i64 i,
-                                                                           const u32 (&mag)[NW], bool neg, i64 ein) {
-    u32 r[L];
-    i64 er;
-    if (!round_mag<L>(mag, ein, r, &er)) neg = false;
-    store_signed<L>(m, plane, i, r, neg);
-    e[i] = er;
-}
 
 // Batched product of aligned operands: C[b, i, j] = sum_k A[b, i, k] B[b, k, j] with A rows and B
 // columns already aligned (k_align); exact accumulation, one rounding.  C is contiguous (b, i, j).
@@ -674,105 +638,131 @@ __global__ void __launch_bounds__(kCauchyThreads, 4) k_cauchy4(const int32_t* __
 }
 
 // ------------------------------------------------------------------------------------------------
-// The pole kernels keep their 2 L + 2 accumulator limbs in shared memory (one column per thread), so that only
-// the operands live in registers: more resident warps to hide the latency of the multiply-add chains.
+// One output of the pole step: sum_j C[j] X[j] over S aligned products (C row aligned, X aligned here to E), rounded once.
+// First try: the product columns from C0 = trunc_cols up, in an accumulator of L + 7 limbs (bits from 32 C0) in shared
+// memory (one column per thread), so that only the operands live in registers.  It lies within 2^(32 (C0 + 2)) of the exact
+// sum; where round_safe shows that no value that close rounds differently, its rounding is the exact sum's.  Elsewhere
+// (heavy cancellation, a sum at a rounding midpoint, exact zeros) exact_dot redoes the sum.  Bound by the integer
+// multiply-add (IMAD.WIDE at half rate: 28 MACs per clock and SM measured) and its latency.  With the 2 L + 2 limbs of
+// the whole sum rounded in registers and the redo unrolled in place the kernels held 168 registers and spilled, three
+// blocks per SM: per 1280-bit task 54.1 ms against 48.8 now, one lambda order at 1024 bits 6.9 against 5.9.
 constexpr int kPoleThreads = 128;
 
-// Pole step, stage 1: Y[t, a, b0, k] = sum_b R[b0, b] H[t_hrow[t], a, b, k]  (R = Rtab[t_R[t]] aligned
-// per row; H aligned per column (a, k) over b here).  Y: (T, S, S, B) contiguous.
+template <int L> B3D_CX int pole_win() { return 2 * L + 2 - trunc_cols<L>(); }    // limbs of the first try's accumulator
+
+// the exact sum (the rare redo), rounded and stored at element oo: a call with loops, out of the way of the kernels' registers
 template <int L>
-__global__ void __launch_bounds__(kPoleThreads, 3) k_pole1(const int32_t* __restrict__ hm, const i64* __restrict__ he, i64 hplane,
+__device__ __noinline__ void exact_dot(const int32_t* cm, i64 cplane, i64 co, const int32_t* xm, const i64* xe, i64 xplane, i64 xo,
+                                       i64 jst, int S, i64 E, i64 Er, int32_t* om, i64* oe, i64 oplane, i64 oo) {
+    constexpr int NW = 2 * L + 2;
+    u32 acc[NW];
+    zero(acc);
+    for (int j = 0; j < S; j++) {
+        u32 c[L], x[L], y[L], prod[NW];
+        const bool nc = load_mag<L>(cm, cplane, co + j, c), nx = load_mag<L>(xm, xplane, xo + j * jst, x);
+        const i64 ex = xe[xo + j * jst];
+        if (is_zero(c) || is_zero(x) || ex == EZ || E - ex >= 32 * L) continue;
+        shr(x, (int)(E - ex), y);
+        zero(prod);
+#pragma unroll 1
+        for (int k = 0; k < L; k++) {
+            u64 cy = 0;
+#pragma unroll 1
+            for (int m = 0; m < L; m++) {
+                cy += (u64)c[k] * y[m] + prod[k + m];
+                prod[k + m] = (u32)cy;
+                cy >>= 32;
+            }
+            prod[k + L] = (u32)cy;
+        }
+        if (nc != nx) sub_borrow(acc, acc, prod, 0u);
+        else add_carry(acc, acc, prod, 0u);
+    }
+    store_rounded<L, NW>(om, oe, oplane, oo, acc, E + Er);
+}
+
+template <int L>
+__device__ __forceinline__ void pole_dot(u32* acc, const int32_t* cm, i64 cplane, i64 co, i64 Er, const int32_t* xm, const i64* xe,
+                                         i64 xplane, i64 xo, i64 jst, int S, int32_t* om, i64* oe, i64 oplane, i64 oo) {
+    constexpr int C0 = trunc_cols<L>(), NWF = pole_win<L>();
+    i64 E = EZ;
+    for (int j = 0; j < S; j++) {
+        const i64 ix = xo + j * jst, ex = xe[ix];
+        if (ex > E && xm[(L - 1) * xplane + ix] != 0) E = ex;
+    }
+    u32 w[NWF];
+    bool any = false;
+    if (E != EZ && Er != EZ) {
+#pragma unroll
+        for (int k = 0; k < NWF; k++) acc[k * kPoleThreads] = 0;
+#pragma unroll 1
+        for (int j = 0; j < S; j++) {
+            const i64 ix = xo + j * jst, ex = xe[ix];
+            u32 y[L], c[L];
+            bool nx;
+            {
+                u32 x[L];
+                nx = load_mag<L>(xm, xplane, ix, x);
+                if (is_zero(x) || ex == EZ || E - ex >= 32 * L) continue;
+                shr(x, (int)(E - ex), y);
+            }
+            const bool nc = load_mag<L>(cm, cplane, co + j, c);
+            if (is_zero(c)) continue;
+            mac_signed_win<L, NWF, C0>(acc, kPoleThreads, c, y, nc != nx);
+            any = true;
+        }
+    }
+    if (!any) {
+#pragma unroll
+        for (int k = 0; k < L; k++) om[k * oplane + oo] = 0;
+        oe[oo] = EZ;
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < NWF; k++) w[k] = acc[k * kPoleThreads];
+    const bool neg = (w[NWF - 1] >> 31) != 0;
+    if (neg) negate(w);
+    if (C0 == 0 || round_safe<L, NWF, (C0 > 0 ? 2 : 0)>(w)) {
+        u32 r[L];
+        i64 er;
+        const bool nz = round_mag<L>(w, E + Er + 32 * C0, r, &er);
+        store_signed<L>(om, oplane, oo, r, neg && nz);
+        oe[oo] = er;
+    } else {
+        exact_dot<L>(cm, cplane, co, xm, xe, xplane, xo, jst, S, E, Er, om, oe, oplane, oo);
+    }
+}
+
+// Pole step, stage 1: Y[t, a, b0, k] = sum_b R[b0, b] H[t_hrow[t], a, b, k]  (R = Rtab[t_R[t]] aligned
+// per row; H aligned per column (a, k) over b).  Y: (T, S, S, B) contiguous.
+template <int L>
+__global__ void __launch_bounds__(kPoleThreads, 4) k_pole1(const int32_t* __restrict__ hm, const i64* __restrict__ he, i64 hplane,
                         const int32_t* __restrict__ Rm, const i64* __restrict__ Re, i64 Rplane,
                         const i64* __restrict__ t_hrow, const i64* __restrict__ t_R, i64 T, i64 B, int S,
                         int32_t* __restrict__ ym, i64* __restrict__ ye, i64 yplane) {
-    i64 idx = blockIdx.x * (i64)blockDim.x + threadIdx.x;
+    extern __shared__ u32 pole_acc[];                    // (pole_win, blockDim.x): this thread's column
+    const i64 idx = blockIdx.x * (i64)blockDim.x + threadIdx.x;
     if (idx >= T * S * S * B) return;
-    i64 k = idx % B, b0 = (idx / B) % S, a = (idx / (B * S)) % S, t = idx / (B * S * S);
-    i64 hrow = t_hrow[t], rk = t_R[t];
-    i64 hb = hrow * S * S * B + a * S * B + k;          // H[hrow, a, b, k] at hb + b * B
-    i64 E = EZ;
-    for (int b = 0; b < S; b++) {
-        i64 ix = hb + b * B;
-        i64 eb = he[ix];
-        if (eb > E && hm[(L - 1) * hplane + ix] != 0) E = eb;
-    }
-    i64 Er = Re[rk * S + b0];
-    constexpr int NW = 2 * L + 2;
-    extern __shared__ u32 pole_acc[];                    // (NW, blockDim.x): this thread's column
-    u32* acc = pole_acc + threadIdx.x;
-    auto sum = [&](auto cols) {                          // acc = the sum from product column cols up
-#pragma unroll
-        for (int w = 0; w < NW; w++) acc[w * kPoleThreads] = 0;
-        bool any = false;
-        if (E != EZ && Er != EZ) {
-#pragma unroll 1
-            for (int b = 0; b < S; b++) {
-                u32 x[L], y[L], r[L];
-                bool nr = load_mag<L>(Rm, Rplane, (rk * S + b0) * S + b, r);
-                if (is_zero(r)) continue;
-                i64 ix = hb + b * B;
-                bool nx = load_mag<L>(hm, hplane, ix, x);
-                i64 ex = he[ix];
-                if (is_zero(x) || ex == EZ || E - ex >= 32 * L) continue;
-                shr(x, (int)(E - ex), y);
-                mac_signed_mem<L, NW, decltype(cols)::value>(acc, kPoleThreads, r, y, nr != nx);
-                any = true;
-            }
-        }
-        return any;
-    };
-    u32 mag[NW];
-    const bool neg = exact_sum<L, NW>(sum, acc, kPoleThreads, mag);
-    store_rounded_mag<L, NW>(ym, ye, yplane, idx, mag, neg, (E == EZ || Er == EZ) ? EZ : E + Er);
+    const i64 k = idx % B, b0 = (idx / B) % S, a = (idx / (B * S)) % S, t = idx / (B * S * S);
+    const i64 rk = t_R[t];
+    pole_dot<L>(pole_acc + threadIdx.x, Rm, Rplane, (rk * S + b0) * S, Re[rk * S + b0], hm, he, hplane,
+                t_hrow[t] * S * S * B + a * S * B + k, B, S, ym, ye, yplane, idx);
 }
 
 // Pole step, stage 2: res[t_slot[t], a0, b0, k] = sum_a QL[a0, a] Y[t, a, b0, k]  (QL = QLtab[t_qL[t]]
-// aligned per row; Y aligned per column (b0, k) over a here).
+// aligned per row; Y aligned per column (b0, k) over a).
 template <int L>
-__global__ void __launch_bounds__(kPoleThreads, 3) k_pole2(const int32_t* __restrict__ ym, const i64* __restrict__ ye, i64 yplane,
+__global__ void __launch_bounds__(kPoleThreads, 4) k_pole2(const int32_t* __restrict__ ym, const i64* __restrict__ ye, i64 yplane,
                         const int32_t* __restrict__ Qm, const i64* __restrict__ Qe, i64 Qplane,
                         const i64* __restrict__ t_qL, const i64* __restrict__ t_slot, i64 T, i64 B, int S,
                         int32_t* __restrict__ rm, i64* __restrict__ re, i64 rplane) {
-    i64 idx = blockIdx.x * (i64)blockDim.x + threadIdx.x;
+    extern __shared__ u32 pole_acc[];                    // (pole_win, blockDim.x): this thread's column
+    const i64 idx = blockIdx.x * (i64)blockDim.x + threadIdx.x;
     if (idx >= T * S * S * B) return;
-    i64 k = idx % B, b0 = (idx / B) % S, a0 = (idx / (B * S)) % S, t = idx / (B * S * S);
-    i64 qk = t_qL[t];
-    i64 yb = t * S * S * B + b0 * B + k;                // Y[t, a, b0, k] at yb + a * S * B
-    i64 E = EZ;
-    for (int a = 0; a < S; a++) {
-        i64 ix = yb + a * S * B;
-        i64 ea = ye[ix];
-        if (ea > E && ym[(L - 1) * yplane + ix] != 0) E = ea;
-    }
-    i64 Eq = Qe[qk * S + a0];
-    constexpr int NW = 2 * L + 2;
-    extern __shared__ u32 pole_acc[];                    // (NW, blockDim.x): this thread's column
-    u32* acc = pole_acc + threadIdx.x;
-    auto sum = [&](auto cols) {                          // acc = the sum from product column cols up
-#pragma unroll
-        for (int w = 0; w < NW; w++) acc[w * kPoleThreads] = 0;
-        bool any = false;
-        if (E != EZ && Eq != EZ) {
-#pragma unroll 1
-            for (int a = 0; a < S; a++) {
-                u32 x[L], y[L], q[L];
-                bool nq = load_mag<L>(Qm, Qplane, (qk * S + a0) * S + a, q);
-                if (is_zero(q)) continue;
-                i64 ix = yb + a * S * B;
-                bool nx = load_mag<L>(ym, yplane, ix, x);
-                i64 ex = ye[ix];
-                if (is_zero(x) || ex == EZ || E - ex >= 32 * L) continue;
-                shr(x, (int)(E - ex), y);
-                mac_signed_mem<L, NW, decltype(cols)::value>(acc, kPoleThreads, q, y, nq != nx);
-                any = true;
-            }
-        }
-        return any;
-    };
-    u32 mag[NW];
-    const bool neg = exact_sum<L, NW>(sum, acc, kPoleThreads, mag);
-    i64 out = t_slot[t] * S * S * B + (a0 * S + b0) * B + k;
-    store_rounded_mag<L, NW>(rm, re, rplane, out, mag, neg, (E == EZ || Eq == EZ) ? EZ : E + Eq);
+    const i64 k = idx % B, b0 = (idx / B) % S, a0 = (idx / (B * S)) % S, t = idx / (B * S * S);
+    const i64 qk = t_qL[t];
+    pole_dot<L>(pole_acc + threadIdx.x, Qm, Qplane, (qk * S + a0) * S, Qe[qk * S + a0], ym, ye, yplane,
+                t * S * S * B + b0 * B + k, S * B, S, rm, re, rplane, t_slot[t] * S * S * B + (a0 * S + b0) * B + k);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1211,7 +1201,7 @@ int Launch<L>::pole(const int32_t* hm, const i64* he, i64 hplane, const int32_t*
                     int32_t* rm, i64* re, i64 rplane, cudaStream_t st) {
     i64 n = T * S * S * B;
     if (n == 0) return 0;
-    const int smem = (2 * L + 2) * kPoleThreads * 4;   // <= 44 KB (L = 42): no opt-in
+    const int smem = pole_win<L>() * kPoleThreads * 4;  // <= 27 KB (L = 46)
     k_pole1<L><<<grid_for(n, kPoleThreads), kPoleThreads, smem, st>>>(hm, he, hplane, Rm, Re, Rplane, t_hrow, t_R, T, B, S,
                                                                        ym, ye, yplane);
     k_pole2<L><<<grid_for(n, kPoleThreads), kPoleThreads, smem, st>>>(ym, ye, yplane, Qm, Qe, Qplane, t_qL, t_slot, T, B,

@@ -404,6 +404,31 @@ template <int L, int NW, int C0 = 0> B3D_HD void mac_signed_mem(u32* acc, int st
     }
 }
 
+// mac_signed_mem with columns below C0 dropped and an accumulator that starts there: limb C0 + k at acc[k * stride], NW limbs
+template <int L, int NW, int C0> B3D_HD void mac_signed_win(u32* acc, int stride, const u32 (&a)[L], const u32 (&b)[L],
+                                                            bool negative) {
+    u32 c0 = 0, c1 = 0, c2 = 0;
+    i64 rc = 0;
+#pragma unroll
+    for (int col = C0; col < 2 * L; col++) {
+#pragma unroll
+        for (int x = 0; x < L; x++) {
+            int y = col - x;
+            if (y >= 0 && y < L) mac96(c0, c1, c2, a[x], b[y]);
+        }
+        i64 r = (i64)acc[(col - C0) * stride] + (negative ? -(i64)c0 : (i64)c0) + rc;
+        acc[(col - C0) * stride] = (u32)r;
+        rc = r >> 32;
+        c0 = c1; c1 = c2; c2 = 0;
+    }
+#pragma unroll
+    for (int k = 2 * L - C0; k < NW; k++) {
+        i64 r = (i64)acc[k * stride] + rc;
+        acc[k * stride] = (u32)r;
+        rc = r >> 32;
+    }
+}
+
 // mac_signed_mem for an a whose limbs below X0 are zero: the same result from (L - X0) L products
 template <int L, int NW, int X0> B3D_HD void mac_signed_high(u32* acc, int stride, const u32 (&a)[L], const u32 (&b)[L],
                                                              bool negative) {

@@ -132,39 +132,6 @@ __device__ __forceinline__ int pm_coff(const PoleMmaArgs& a, int n) {
 
 __device__ __forceinline__ int pm_jst(const PoleMmaArgs& a) { return a.stage == 1 ? (int)a.B : a.S * (int)a.B; }
 
-// the exact sum of output (row i, column n) of an item from the operands in memory, rounded once and stored (the rare redo):
-// xo, co, oo: element offsets of X[j = 0], C[i, 0] and the output
-template <int L>
-__device__ __noinline__ void pm_exact(const PoleMmaArgs& a, i64 xo, i64 co, i64 oo, i64 E, i64 Er) {
-    constexpr int NW = 2 * L + 2;
-    const int jst = pm_jst(a);
-    u32 acc[NW];
-    zero(acc);
-    for (int j = 0; j < a.S; j++) {
-        u32 c[L], x[L], y[L];
-        const bool nc = load_mag<L>(a.cm, a.cplane, co + j, c), nx = load_mag<L>(a.xm, a.xplane, xo + (i64)j * jst, x);
-        const i64 ex = a.xe[xo + (i64)j * jst];
-        if (is_zero(c) || is_zero(x) || ex == EZ || E - ex >= 32 * L) continue;
-        shr(x, (int)(E - ex), y);
-        u32 prod[NW];                                               // schoolbook rows: a loop, not an unrolled product
-        zero(prod);
-#pragma unroll 1
-        for (int k = 0; k < L; k++) {
-            u64 cy = 0;
-#pragma unroll 1
-            for (int m = 0; m < L; m++) {
-                cy += (u64)c[k] * y[m] + prod[k + m];
-                prod[k + m] = (u32)cy;
-                cy >>= 32;
-            }
-            prod[k + L] = (u32)cy;
-        }
-        if (nc != nx) sub_borrow(acc, acc, prod, 0u);
-        else add_carry(acc, acc, prod, 0u);
-    }
-    store_rounded<L, NW>(a.om, a.oe, a.oplane, oo, acc, E + Er);
-}
-
 // one column of a row: its positions d4 from P0 -> limbs (two's complement, one more for the sign)
 template <int L>
 __device__ __forceinline__ i64 pm_limbs(const int4* d4, u32 (&w)[PoleMmaGeom<L>::NPW + 1]) {
@@ -235,7 +202,7 @@ __device__ __forceinline__ void pm_column(const PoleMmaArgs& a, u32 (&w)[PoleMma
         }
     }
     if (!done) {
-        pm_exact<L>(a, xo, co, oo, E, Er);
+        exact_dot<L>(a.cm, a.cplane, co, a.xm, a.xe, a.xplane, xo, pm_jst(a), a.S, E, Er, a.om, a.oe, a.oplane, oo);
         return;
     }
     store_signed<L>(a.om, a.oplane, oo, r, neg && er != EZ);
