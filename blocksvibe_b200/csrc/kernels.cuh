@@ -883,45 +883,22 @@ __global__ void __launch_bounds__(kMomThreads, 3) k_moments_stage(const int32_t*
     ye[out] = ey;
 }
 
-// One thread per (row, column) item, the moment orders in chunks of kFlushKC: for each staged term, the exact
-// product |Y| n^k0 (n^k0 from the table nk: nk[(k * NN + n) * KW + j], 32-bit limbs; nkb[k * NN + n] its bit
-// length), then times n for each further order of the chunk, each added into that order's accumulator (a
-// shared-memory column of L + 3 words, two's complement) at the word and bit offset of its exponent: no barrel
-// shifter, one funnel shift per word.  The accumulator of order k keeps the bits from 32 (L + 2) below the bound
-// E_k = max_w (e_w + NB + bits(n_w^k)) of its terms (truncated below), then rounds once.
+// One thread per (row, column) item, the moment orders in chunks of kFlushKC.  Each staged term is shifted once per chunk
+// onto one grid for all levels and orders, in two's complement, multiplied by n^k0 (the table nk: nk[(k * NN + n) * KW + j],
+// 32-bit limbs; nkb[k * NN + n] its bit length) and then by n from order to order, modulo 2^(32 NA): every addition into an
+// order's accumulator (a shared-memory column of NA words) is the same straight carry chain, whatever the term's sign
+// and exponent.  The grid reaches 32 (LO + 2 + KW) bits below E, the exponent above the chunk's largest term with n^k != 0,
+// and KW + 1 words above it: a term is truncated (towards zero) below 2^(E - 32 (LO + 2)) even after its product with
+// n^k < 2^(32 KW), and |sum| < W 2^(32 KW) 2^E.  A term with n = 0 counts for order 0 only, which then is a chunk
+// of its own.  One rounding per order.
+// Bound by the latency of the carry chains at the eight warps per SM that shared memory leaves room for: the sum of one order
+// and the product for the next run side by side (10.0 ms one after the other; chunks of three orders 8.6, of two 9.4).
+// Before, every word and order had its own offset, bounds check and carry by comparison: 1024 bits, R = 11, W = 40, 593,400 full
+// columns 19.7 ms, now 8.1; 1280 bits, R = 27, 170,000 columns: W = 72 43.5 and 20.1, a second window of W = 8 6.4 and 3.7.
 constexpr int kFlushThreads = 64;
 constexpr int kFlushKC = 4;
 
-template <int ACC, int NP>
-__device__ __forceinline__ void add_at_offset(u32* acc, int stride, const u32 (&P)[NP], i64 off, bool neg) {
-    const i64 qq = off >= 0 ? off / 32 : -((-off + 31) / 32);      // floor(off / 32)
-    const int f = (int)(off - 32 * qq);
-    const int q = (int)qq;
-    u32 carry = 0;                                                  // carry (add) or borrow (subtract)
-#pragma unroll
-    for (int j = 0; j <= NP; j++) {
-        const int a = j + q;
-        const u32 lo = j > 0 ? P[j - 1] : 0u, hi = j < NP ? P[j] : 0u;
-        const u32 v = fsl(lo, hi, f);                               // word j of P 2^f
-        if (a < 0 || a >= ACC) continue;                            // below the accumulator: truncated
-        const u32 w = acc[a * stride];
-        if (!neg) {
-            const u32 s1 = w + v, s2 = s1 + carry;
-            carry = (s1 < w) | (s2 < s1);
-            acc[a * stride] = s2;
-        } else {
-            const u32 d1 = w - v, d2 = d1 - carry;
-            carry = (w < v) | (d1 < carry);
-            acc[a * stride] = d2;
-        }
-    }
-    for (int a = NP + 1 + q; carry && a < ACC; a++) {              // propagate to the top
-        if (a < 0) continue;
-        const u32 w = acc[a * stride];
-        if (!neg) { acc[a * stride] = w + 1; carry = w == 0xFFFFFFFFu; }
-        else { acc[a * stride] = w - 1; carry = w == 0u; }
-    }
-}
+B3D_CX int flush_words(int LO, int KW) { return LO + 2 * KW + 3; }
 
 template <int L, int LO, int KW, bool ACCUMULATE>
 __global__ void __launch_bounds__(kFlushThreads) k_moments_flush(const int32_t* __restrict__ ym, const i64* __restrict__ ye,
@@ -929,87 +906,109 @@ __global__ void __launch_bounds__(kFlushThreads) k_moments_flush(const int32_t* 
                           const u32* __restrict__ nk, const int32_t* __restrict__ nkb, int NN,
                           int32_t* __restrict__ mm, i64* __restrict__ me, i64 mplane, bool zero_rows) {
     constexpr int NB = nb_bits(L);                       // staged terms: L limbs; moments: LO limbs
-    constexpr int ACC = LO + 3;
-    constexpr int NP = L + KW + 1;                       // |Y| n^k, k within a chunk: n^k0 < 2^(32 KW), n^3 < 2^32
-    extern __shared__ u32 flush_acc[];                   // (kFlushKC * ACC, blockDim.x)
+    constexpr int NA = flush_words(LO, KW), BELOW = 32 * (LO + 2 + KW);
+    extern __shared__ u32 flush_acc[];                   // (kFlushKC * NA, blockDim.x)
     const i64 item = blockIdx.x * (i64)blockDim.x + threadIdx.x;
     if (item >= rows * N) return;
     const i64 row = item / N, c = item - row * N;
-    const i64 sh = row_shift[row];
-    if (zero_rows && m0 + sh > 0) return;                // only the rows with n = 0 in the window
+    const i64 n0 = m0 + row_shift[row];
+    if (zero_rows && n0 > 0) return;                     // only the rows with n = 0 in the window
     u32* acc = flush_acc + threadIdx.x;
-    for (int k0 = 0; k0 < R1; k0 += kFlushKC) {
-        const int kc = R1 - k0 < kFlushKC ? R1 - k0 : kFlushKC;
-        i64 E[kFlushKC];
-#pragma unroll
-        for (int kk = 0; kk < kFlushKC; kk++) E[kk] = EZ;
+    for (int k0 = 0, kc; k0 < R1; k0 += kc) {
+        kc = R1 - k0 < kFlushKC ? R1 - k0 : kFlushKC;
+        if (k0 == 0 && n0 <= 0) kc = 1;
+        i64 E = EZ;                                      // above every term: |Y| < 2^(ey + NB)
         for (int w = 0; w < W; w++) {
-            const i64 ey = ye[(w * rows + row) * N + c];
-            const i64 n = m0 + w + sh;
-            if (ey == EZ || n >= NN) continue;
-#pragma unroll
-            for (int kk = 0; kk < kFlushKC; kk++) {
-                if (kk >= kc) break;
-                const int kb = nkb[(k0 + kk) * NN + n];
-                if (kb && ey + NB + kb > E[kk]) E[kk] = ey + NB + kb;
-            }
+            const i64 ey = ye[(w * rows + row) * N + c], n = n0 + w;
+            if (ey != EZ && n < NN && nkb[k0 * NN + n] != 0 && ey + NB > E) E = ey + NB;
         }
-        for (int k = 0; k < kFlushKC * ACC; k++) acc[k * kFlushThreads] = 0;
+        if (E == EZ) {
+            for (int kk = 0; kk < kc && !ACCUMULATE; kk++) {
+                const i64 o = (row * R1 + k0 + kk) * N + c;
+#pragma unroll
+                for (int k = 0; k < LO; k++) mm[k * mplane + o] = 0;
+                me[o] = EZ;
+            }
+            continue;
+        }
+        for (int k = 0; k < kc * NA; k++) acc[k * kFlushThreads] = 0;
         for (int w = 0; w < W; w++) {
             const i64 ix = (w * rows + row) * N + c;
-            const i64 ey = ye[ix];
-            const i64 n = m0 + w + sh;
-            if (ey == EZ || n >= NN) continue;
-            u32 y[L];
-            const bool neg = load_mag<L>(ym, yplane, ix, y);
-            u32 P[NP];
-            zero(P);
+            const i64 ey = ye[ix], n = n0 + w;
+            if (ey == EZ || n >= NN || nkb[k0 * NN + n] == 0) continue;
+            const i64 off = BELOW - (E - ey);            // bit of the grid that bit 0 of Y falls on
+            if (off <= -32 * L) continue;
+            const int q = (int)(off >= 0 ? off >> 5 : -((-off + 31) >> 5)), f = (int)off - 32 * q;
+            const int32_t* y = ym + ix;
+            const u32 sign = y[(L - 1) * yplane] < 0 ? 0xFFFFFFFFu : 0u;
+            u32 u[NA];
+            {
+                // grid word j = limbs j - q - 1 and j - q of Y by f bits; limbs above Y are its sign
+                u32 prev = q < 0 ? (u32)y[(-q - 1) * yplane] : 0u;
+                const int32_t* yj = y - q * yplane;
 #pragma unroll
-            for (int j = 0; j < KW; j++) {               // P = |Y| n^k0
-                const u32 b = nk[((i64)k0 * NN + n) * KW + j];
-                u32 carry = 0;
-#pragma unroll
-                for (int i = 0; i < L; i++) {
-                    const u64 v = (u64)y[i] * b + P[i + j] + carry;
-                    P[i + j] = (u32)v;
-                    carry = (u32)(v >> 32);
+                for (int j = 0; j < NA; j++) {
+                    u32 cur = j - q < 0 ? 0u : sign;
+                    if ((unsigned)(j - q) < (unsigned)L) cur = (u32)yj[j * yplane];
+                    u[j] = fsl(prev, cur, f);
+                    prev = cur;
                 }
-                P[L + j] += carry;
             }
+            if (off < 0 && sign) {                       // bits cut off a negative term: towards zero, so one up
+                const int whole = f ? -q - 1 : -q;       // limbs cut off whole, and the low 32 - f bits of the next
+                u32 cut = f ? (u32)y[whole * yplane] << f : 0u;
+                for (int i = 0; i < whole; i++) cut |= (u32)y[i * yplane];
+                if (cut) add_bit(u, u, 1u);
+            }
+            if (k0 > 0) {                                // u *= n^k0
+                u32 P[NA];
+                const u32* b = nk + ((i64)k0 * NN + n) * KW;
+                const int nw = (nkb[k0 * NN + n] + 31) >> 5;
+                mul_small(P, u, b[0]);
+#pragma unroll
+                for (int j = 1; j < KW; j++) {
+                    if (j >= nw) break;
+                    u32 t[NA];
+                    mul_small(t, u, b[j]);
+#pragma unroll
+                    for (int i = NA - 1; i >= 0; i--) t[i] = i >= j ? t[i - j] : 0u;
+                    add_carry(P, P, t, 0u);
+                }
+#pragma unroll
+                for (int j = 0; j < NA; j++) u[j] = P[j];
+            }
+            u32* a = acc;
 #pragma unroll 1
-            for (int kk = 0; kk < kc; kk++) {
-                if (kk > 0) {                            // P *= n (exact)
-                    u32 carry = 0;
+            for (int kk = 1; kk < kc; kk++, a += NA * kFlushThreads) {   // the order's sum, and u *= n for the next
+                u32 s[NA], v[NA];
 #pragma unroll
-                    for (int i = 0; i < NP; i++) {
-                        const u64 v = (u64)P[i] * (u64)n + carry;
-                        P[i] = (u32)v;
-                        carry = (u32)(v >> 32);
-                    }
+                for (int j = 0; j < NA; j++) s[j] = a[j * kFlushThreads];
+                add_mul_small(s, v, u, (u32)n);
+#pragma unroll
+                for (int j = 0; j < NA; j++) {
+                    a[j * kFlushThreads] = s[j];
+                    u[j] = v[j];
                 }
-                if (E[kk] == EZ || nkb[(k0 + kk) * NN + n] == 0) continue;
-                add_at_offset<ACC, NP>(acc + kk * ACC * kFlushThreads, kFlushThreads, P, ey - (E[kk] - 32 * (LO + 2)), neg);
             }
+            u32 s[NA];
+#pragma unroll
+            for (int j = 0; j < NA; j++) s[j] = a[j * kFlushThreads];
+            add_carry(s, s, u, 0u);
+#pragma unroll
+            for (int j = 0; j < NA; j++) a[j * kFlushThreads] = s[j];
         }
+#pragma unroll 1
         for (int kk = 0; kk < kc; kk++) {
             const i64 o = (row * R1 + k0 + kk) * N + c;
-            if (E[kk] == EZ) {
-                if (!ACCUMULATE) {
+            u32 mag[NA];
 #pragma unroll
-                    for (int k = 0; k < LO; k++) mm[k * mplane + o] = 0;
-                    me[o] = EZ;
-                }
-                continue;
-            }
-            u32 mag[ACC];
-#pragma unroll
-            for (int k = 0; k < ACC; k++) mag[k] = acc[(kk * ACC + k) * kFlushThreads];
-            const bool negs = (mag[ACC - 1] >> 31) != 0;
+            for (int k = 0; k < NA; k++) mag[k] = acc[(kk * NA + k) * kFlushThreads];
+            const bool negs = (mag[NA - 1] >> 31) != 0;
             if (negs) negate(mag);
             u32 r[LO];
             i64 er;
             bool nr = negs;
-            if (!round_mag<LO>(mag, E[kk] - 32 * (LO + 2), r, &er)) nr = false;
+            if (!round_mag<LO>(mag, E - BELOW, r, &er)) nr = false;
             if (ACCUMULATE) {
                 u32 v[LO], sum[LO];
                 const bool nv = load_mag<LO>(mm, mplane, o, v);
@@ -1239,7 +1238,7 @@ int Launch<L>::moments_flush(const int32_t* ym, const i64* ye, i64 yplane, const
     if (items == 0 || W == 0) return 0;
     const unsigned grid = (unsigned)((items + kFlushThreads - 1) / kFlushThreads);
 #define B3D_FLUSH(LOC, KWC, AC) do {                                                                       \
-        const int smem = kFlushThreads * kFlushKC * ((LOC) + 3) * 4;     /* above 48 KB from 46 limbs: opt in */ \
+        const int smem = kFlushThreads * kFlushKC * flush_words(LOC, KWC) * 4;   /* above 48 KB: opt in */           \
         static unsigned long long opted = 0;                /* devices whose limit is raised */                  \
         const unsigned long long dbit = device_bit();                                                            \
         if (!(opted & dbit) || !dbit) {                                                                          \

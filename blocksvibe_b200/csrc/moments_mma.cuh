@@ -19,9 +19,9 @@
 //
 // What bounds it: latency and integer issue of the limb work around the MMAs (per four columns of R = 11, W = 40: digits
 // 11 K clocks, TMEM to limbs 13 K, sums and rounding 14 K, stores 4 K, the tensor pipe 5 % busy, two CTAs per SM).  The
-// cost of a column hardly depends on R and W, that of k_moments_flush is W R1 times some 400 instructions, hence the rule
-// of flush(): per 1280-bit task (R = 27, W = 72) 25.4 ms against 51.3; 896 bits, R = 6, W = 32, few columns 0.21 against
-// 0.56; 1024 bits, R = 11, W = 40, 593,400 columns 11.9 against 11.7 (k_moments_flush stays).
+// cost of a column grows with R but hardly with W, that of k_moments_flush with W R1, hence the rule of flush(): 1280 bits, R = 27,
+// 170,000 columns: W = 72 12.1 ms against 20.3, W = 32 8.6 against 8.9; 1024 bits, R = 15, W = 48, 300,000 columns 10.6 against
+// 8.3; R = 11, W = 40, 593,400 columns 13.1 against 8.5, 12,500 columns 0.28 against 0.37.
 #pragma once
 #include <atomic>
 #include <cmath>
@@ -421,9 +421,15 @@ __global__ void __launch_bounds__(kFlushMmaThreads, 2) k_moments_flush_mma(Flush
 
 #endif
 
-// Which form: the tensor cores from W R1 = 600 on (both forms cost the same at 480, above), or where the columns do not
-// fill the CUDA-core form's thread per column (148 SMs x 8 blocks x 64), from ten levels on.
-inline bool flush_mma_pays(int W, int R1, i64 cols) { return W >= 10 && ((i64)W * R1 >= 600 || cols < 148 * 8 * 64); }
+// Which form, by times of both on a B200 (milliseconds, tensor cores / CUDA cores).  Many columns: the tensor cores from W R1 = 900
+// (1280 bits: W R1 = 896 8.6 / 8.9, 1344 10.7 / 13.4, 768 7.7 / 8.4; 1024 bits: 768 10.6 / 8.3).  Columns that leave the CUDA-core
+// form's thread per column short of threads: 1024 bits, W R1 = 480: 12,500 columns 0.28 / 0.37, 25,000 0.60 / 0.57; 896
+// bits, 224: 8,000 0.13 / 0.21, 20,000 0.28 / 0.24; the line is at 112 columns per SM, from W R1 = 128 (256 bits, 60: 1,800 columns
+// 0.043 / 0.042, 20,000 0.19 / 0.05).
+inline bool flush_mma_pays(int W, int R1, i64 cols) {
+    const i64 terms = (i64)W * R1;
+    return terms >= 900 || (W >= 10 && terms >= 128 && cols < 148 * 112);
+}
 
 template <int L>
 struct FlushMmaLaunch {

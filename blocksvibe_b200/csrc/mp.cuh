@@ -207,6 +207,42 @@ template <int N> B3D_HD u32 add_bit(u32 (&r)[N], const u32 (&a)[N], u32 c) {
     return add_carry(r, a, z, c);
 }
 
+// r = a b mod 2^(32 N) (two's complement a as well): the products of the even and of the odd limbs, which do not overlap among
+// themselves, added in one carry chain.  r may be a.
+template <int N> B3D_HD void split_products(const u32 (&a)[N], u32 b, u32 (&e)[N], u32 (&o)[N]) {
+    o[0] = 0;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const u64 p = (u64)a[k] * b;
+        u32* t = k & 1 ? o : e;
+        t[k] = (u32)p;
+        if (k + 1 < N) t[k + 1] = (u32)(p >> 32);
+    }
+}
+
+template <int N> B3D_HD void mul_small(u32 (&r)[N], const u32 (&a)[N], u32 b) {
+    u32 e[N], o[N];
+    split_products(a, b, e, o);
+    add_carry(r, e, o, 0u);
+}
+
+// s += a and r = a b, their two carry chains side by side (either alone is bound by the latency of its carries)
+template <int K, int N> B3D_HD void add_mul_from(u32 (&s)[N], u32 (&r)[N], const u32 (&a)[N], const u32 (&e)[N], const u32 (&o)[N],
+                                                 u32& c, u32& d) {
+    if constexpr (K < N) {
+        constexpr int NC = N - K >= 8 ? 8 : (N - K >= 4 ? 4 : (N - K >= 2 ? 2 : 1));
+        add_carry_chunk<K, NC, N>(s, s, a, c);
+        add_carry_chunk<K, NC, N>(r, e, o, d);
+        add_mul_from<K + NC, N>(s, r, a, e, o, c, d);
+    }
+}
+
+template <int N> B3D_HD void add_mul_small(u32 (&s)[N], u32 (&r)[N], const u32 (&a)[N], u32 b) {
+    u32 e[N], o[N], c = 0, d = 0;
+    split_products(a, b, e, o);
+    add_mul_from<0, N>(s, r, a, e, o, c, d);
+}
+
 // two's complement negation in place
 template <int N> B3D_HD void negate(u32 (&a)[N]) {
     u32 z[N];
