@@ -361,7 +361,7 @@ class Derivs:
         self._stage.e.fill_(mpf.EZ)                      # entries a level does not write read as zero
 
     def check_errors(self):
-        """raise B3DError if the flush gave up a bounded wait (synchronises the device)"""
+        """raise B3DError if the flush gave up a bounded wait (synchronises the device); clears the flag it raises for"""
         code = int(self.err.item())
         if code:
             self.err.zero_()

@@ -29,7 +29,7 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
-from . import mpf
+from . import _lib, mpf, rns
 from .derivatives import Derivs, resize
 from .mpf import MPF
 from .output import Output, apply_per_order
@@ -94,6 +94,12 @@ def task_results(tjs, pp, vals, infos, Smax, L, nq):
             for q in range(nq)]
 
 
+def _raise_codes(codes):
+    if any(codes):
+        raise _lib.B3DError(f"a tensor-core kernel did not complete (pole step {codes[0]}, moments flush {codes[1]}, "
+                            f"residue products {codes[2:]})")
+
+
 class Operator:
     """Plan + recursion constants + derivative constants + write_output maps of one (pp, sign) subgroup,
     built once and reused for every batch (the reference rebuilds them per subgroup: cli.py:401-406)."""
@@ -109,6 +115,16 @@ class Operator:
                           kept_pole_order=group.kept_pole_order, device=device)
         self.outs = {(c, d): Output(c, group.Lambda, parity, d, self.der.Ld, device) for c in coords for d in d12s}
         self.device = torch.device(device)
+
+    def _flags(self):
+        """the device flags of the kernels with bounded waits: pole step, moments flush, residue products"""
+        return torch.cat([self.rec.err, self.der.err] + rns.error_flags(self.device))
+
+    def check_errors(self):
+        """raise B3DError if a kernel of this operator's work gave up a bounded wait: its results are incomplete (waits
+        for the current stream).  Every way of handing results to the host does this.  The flags stay set, as batches on
+        other streams may share them: the operator is used up; the check_errors of rec, der and the rns module clear."""
+        _raise_codes(self._flags().tolist())
 
     def footprint_bytes(self, B):
         return self.rec.footprint_bytes(B) + self.der.footprint_bytes(B) + \
@@ -162,7 +178,8 @@ class Operator:
         return {c: resize(apply_per_order(o, nums), self.L) for (c, dd), o in self.outs.items() if dd == d12}
 
     def to_host(self, outs):
-        """device results -> host limb arrays through reusable pinned buffers (one D2H copy per array)"""
+        """device results -> host limb arrays through reusable pinned buffers (one D2H copy per array); raises
+        B3DError if a kernel did not complete (check_errors)"""
         host = {}
         for c, r in outs.items():
             key = (c, tuple(r.m.shape))
@@ -175,7 +192,7 @@ class Operator:
             buf[0].copy_(r.m, non_blocking=True)
             buf[1].copy_(r.e, non_blocking=True)
             host[c] = buf
-        torch.cuda.current_stream(self.device).synchronize()
+        self.check_errors()                            # waits for the stream, the copies included
         return host
 
 
@@ -208,6 +225,11 @@ class GraphStep:
         self.h.m.copy_(self.stage.m.permute(0, 2, 3, 4, 5, 1))
         self.h.e.copy_(self.stage.e.permute(1, 2, 3, 4, 0))
 
+    def check_errors(self):
+        """raise B3DError if a kernel of a replay gave up a bounded wait (Operator.check_errors; run() does not wait, so
+        a program that reads `out` itself calls this first)"""
+        self.op.check_errors()
+
     def run(self, tasks=None):
         if tasks is not None:
             self.load(tasks)
@@ -222,11 +244,13 @@ class GraphStep:
         host = [{c: (torch.empty(x.m.shape, dtype=torch.int32, pin_memory=True),
                      torch.empty(x.e.shape, dtype=torch.int64, pin_memory=True)) for c, x in self.out.items()}
                 for _ in range(2)]
+        flags = self.op._flags()
+        flags = [(torch.empty_like(flags), torch.empty(flags.shape, dtype=flags.dtype, pin_memory=True)) for _ in range(2)]
         in_ready = [torch.cuda.Event() for _ in range(2)]      # inputs of the slot are on the device
         in_free = [torch.cuda.Event() for _ in range(2)]       # the step has taken them into the static input
         out_ready = [torch.cuda.Event() for _ in range(2)]     # results copied out of the static output
         host_ready = [torch.cuda.Event() for _ in range(2)]    # results on the host; the device copy is free
-        return copy, stage, outd, host, in_ready, in_free, out_ready, host_ready
+        return copy, stage, outd, host, flags, in_ready, in_free, out_ready, host_ready
 
     def run_stream(self, batches):
         """Pipelined replays.  For each list of host tasks (h_inf in pinned memory) taken from `batches`, yields
@@ -235,12 +259,13 @@ class GraphStep:
         batch i's graph runs, so the host transfers overlap the step; the step's stream itself only adds two
         device-to-device copies (inputs into the static buffer, results out of it).  Staging buffers, device
         result copies and host buffers are double-buffered, every reuse ordered by an event; they are allocated on
-        the first call and kept for the next ones."""
+        the first call and kept for the next ones.  Raises B3DError in the place of results whose kernels did not
+        complete (Operator.check_errors)."""
         dev = self.op.device
         main = torch.cuda.current_stream(dev)
         if getattr(self, "_pipe", None) is None:               # built once, reused by every call
             self._pipe = self._pipeline_buffers()
-        copy, stage, outd, host, in_ready, in_free, out_ready, host_ready = self._pipe
+        copy, stage, outd, host, flags, in_ready, in_free, out_ready, host_ready = self._pipe
 
         def bring_in(j, tasks):
             with torch.cuda.stream(copy):
@@ -273,18 +298,22 @@ class GraphStep:
             for c, x in self.out.items():
                 outd[j][c][0].copy_(x.m)
                 outd[j][c][1].copy_(x.e)
+            flags[j][0].copy_(self.op._flags()[:len(flags[j][0])])
             out_ready[j].record(main)
             with torch.cuda.stream(copy):
                 copy.wait_event(out_ready[j])
                 for c in self.out:
                     host[j][c][0].copy_(outd[j][c][0], non_blocking=True)
                     host[j][c][1].copy_(outd[j][c][1], non_blocking=True)
+                flags[j][1].copy_(flags[j][0], non_blocking=True)
                 host_ready[j].record(copy)
             if prev is not None:
                 host_ready[prev].synchronize()
+                _raise_codes(flags[prev][1].tolist())
                 yield host[prev]
             prev, i = j, i + 1
         host_ready[prev].synchronize()
+        _raise_codes(flags[prev][1].tolist())
         yield host[prev]
 
 

@@ -307,7 +307,8 @@ class Recursion:
         return pole_mma_speedup(self.L, self.plan.Smax, B) >= POLE_MIN_GAIN
 
     def check_errors(self):
-        """raise B3DError if a kernel of this recursion gave up a bounded wait (synchronises the device)"""
+        """raise B3DError if a kernel of this recursion gave up a bounded wait (synchronises the device); clears the
+        flag it raises for"""
         code = int(self.err.item())
         if code:
             self.err.zero_()

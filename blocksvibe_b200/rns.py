@@ -275,10 +275,18 @@ def gemm_aligned_rns(Aal, Bal, crt="tensor", lanes=None):
     return MPF(cm.reshape(L, nb, M, N), ce)
 
 
+def error_flags(device):
+    """the device flags (one int32 each) that the tensor-core launches on `device` set when a bounded wait expires"""
+    d = torch.device(device)
+    if d.type == "cuda" and d.index is None:
+        d = torch.device("cuda", torch.cuda.current_device())
+    return [tb.err for tb in list(_TABLES.values()) if tb.err.device == d]
+
+
 def check_errors(device):
-    """raise if a tensor-core launch on `device` recorded a timeout (bounded mbarrier waits)"""
-    for (L, dev), tb in _TABLES.items():
-        if dev == str(device) and int(tb.err.item()) != 0:
-            code = int(tb.err.item())
-            tb.err.zero_()
+    """raise if a tensor-core launch on `device` recorded a timeout (bounded mbarrier waits); clears the flag it raises for"""
+    for err in error_flags(device):
+        code = int(err.item())
+        if code != 0:
+            err.zero_()
             raise _lib.B3DError(f"b3d_rns_mma: a wait timed out (code {code})")

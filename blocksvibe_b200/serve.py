@@ -198,7 +198,7 @@ class Server:
                             hm.copy_(x.m, non_blocking=True)
                             he.copy_(x.e, non_blocking=True)
                             host[c] = (hm, he)
-                    stream.synchronize()
+                    op.check_errors()                      # waits for the stream, the copies included
                 now = time.perf_counter()
                 d12 = head.task.delta_1_plus_2
                 for q, r in enumerate(batch):
