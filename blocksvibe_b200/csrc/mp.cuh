@@ -53,7 +53,7 @@ B3D_HD void mac96(u32& c0, u32& c1, u32& c2, u32 a, u32 b) {
     asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
         "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
         "addc.u32 %2, %2, 0;"
-        : "+r"(c0), "+r"(c1), "+r"(c2) : "r"(a), "r"(b));
+        : "+&r"(c0), "+r"(c1), "+r"(c2) : "r"(a), "r"(b));   // c0 is written before a and b are read again
 #else
     u64 p = (u64)a * b;
     u64 lo = (u64)c0 + (u32)p;
@@ -69,7 +69,8 @@ template <int N> B3D_HD void zero(u32 (&a)[N]) {
 
 // Carry chains.  The carry flag does not survive between asm statements, so a chain runs in statements of eight limbs
 // with the carry in a register between them: 10 instructions per eight limbs against 16 to 32 for carries formed by
-// 64-bit sums or comparisons.
+// 64-bit sums or comparisons.  A statement of several limbs writes its first results before it reads its last operands, so
+// they are early clobbers: no result may take the register of an operand whose life ends here.
 // r = a + b + c (c <= 1); returns the carry out.  r may be a or b.
 template <int K, int NC, int N> B3D_HD void add_carry_chunk(u32 (&r)[N], const u32 (&a)[N], const u32 (&b)[N], u32& c) {
 #ifdef __CUDA_ARCH__
@@ -85,7 +86,7 @@ template <int K, int NC, int N> B3D_HD void add_carry_chunk(u32 (&r)[N], const u
             "addc.cc.u32 %6, %15, %23;\n\t"
             "addc.cc.u32 %7, %16, %24;\n\t"
             "addc.u32 %8, 0, 0;\n\t}"
-            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "=r"(r[K + 4]), "=r"(r[K + 5]), "=r"(r[K + 6]), "=r"(r[K + 7]), "+r"(c)
+            : "=&r"(r[K + 0]), "=&r"(r[K + 1]), "=&r"(r[K + 2]), "=&r"(r[K + 3]), "=&r"(r[K + 4]), "=&r"(r[K + 5]), "=&r"(r[K + 6]), "=&r"(r[K + 7]), "+r"(c)
             : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(a[K + 4]), "r"(a[K + 5]), "r"(a[K + 6]), "r"(a[K + 7]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]), "r"(b[K + 4]), "r"(b[K + 5]), "r"(b[K + 6]), "r"(b[K + 7]));
     } else if constexpr (NC == 4) {
         asm("{\n\t.reg .u32 t;\n\t"
@@ -95,7 +96,7 @@ template <int K, int NC, int N> B3D_HD void add_carry_chunk(u32 (&r)[N], const u
             "addc.cc.u32 %2, %7, %11;\n\t"
             "addc.cc.u32 %3, %8, %12;\n\t"
             "addc.u32 %4, 0, 0;\n\t}"
-            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "+r"(c)
+            : "=&r"(r[K + 0]), "=&r"(r[K + 1]), "=&r"(r[K + 2]), "=&r"(r[K + 3]), "+r"(c)
             : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]));
     } else if constexpr (NC == 2) {
         asm("{\n\t.reg .u32 t;\n\t"
@@ -103,7 +104,7 @@ template <int K, int NC, int N> B3D_HD void add_carry_chunk(u32 (&r)[N], const u
             "addc.cc.u32 %0, %3, %5;\n\t"
             "addc.cc.u32 %1, %4, %6;\n\t"
             "addc.u32 %2, 0, 0;\n\t}"
-            : "=r"(r[K + 0]), "=r"(r[K + 1]), "+r"(c)
+            : "=&r"(r[K + 0]), "=&r"(r[K + 1]), "+r"(c)
             : "r"(a[K + 0]), "r"(a[K + 1]), "r"(b[K + 0]), "r"(b[K + 1]));
     } else {
         asm("{\n\t.reg .u32 t;\n\t"
@@ -150,7 +151,7 @@ template <int K, int NC, int N> B3D_HD void sub_borrow_chunk(u32 (&r)[N], const 
             "subc.cc.u32 %6, %15, %23;\n\t"
             "subc.cc.u32 %7, %16, %24;\n\t"
             "subc.u32 %8, 0, 0;\n\tand.b32 %8, %8, 1;\n\t}"
-            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "=r"(r[K + 4]), "=r"(r[K + 5]), "=r"(r[K + 6]), "=r"(r[K + 7]), "+r"(c)
+            : "=&r"(r[K + 0]), "=&r"(r[K + 1]), "=&r"(r[K + 2]), "=&r"(r[K + 3]), "=&r"(r[K + 4]), "=&r"(r[K + 5]), "=&r"(r[K + 6]), "=&r"(r[K + 7]), "+r"(c)
             : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(a[K + 4]), "r"(a[K + 5]), "r"(a[K + 6]), "r"(a[K + 7]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]), "r"(b[K + 4]), "r"(b[K + 5]), "r"(b[K + 6]), "r"(b[K + 7]));
     } else if constexpr (NC == 4) {
         asm("{\n\t.reg .u32 t;\n\t"
@@ -160,7 +161,7 @@ template <int K, int NC, int N> B3D_HD void sub_borrow_chunk(u32 (&r)[N], const 
             "subc.cc.u32 %2, %7, %11;\n\t"
             "subc.cc.u32 %3, %8, %12;\n\t"
             "subc.u32 %4, 0, 0;\n\tand.b32 %4, %4, 1;\n\t}"
-            : "=r"(r[K + 0]), "=r"(r[K + 1]), "=r"(r[K + 2]), "=r"(r[K + 3]), "+r"(c)
+            : "=&r"(r[K + 0]), "=&r"(r[K + 1]), "=&r"(r[K + 2]), "=&r"(r[K + 3]), "+r"(c)
             : "r"(a[K + 0]), "r"(a[K + 1]), "r"(a[K + 2]), "r"(a[K + 3]), "r"(b[K + 0]), "r"(b[K + 1]), "r"(b[K + 2]), "r"(b[K + 3]));
     } else if constexpr (NC == 2) {
         asm("{\n\t.reg .u32 t;\n\t"
@@ -168,7 +169,7 @@ template <int K, int NC, int N> B3D_HD void sub_borrow_chunk(u32 (&r)[N], const 
             "subc.cc.u32 %0, %3, %5;\n\t"
             "subc.cc.u32 %1, %4, %6;\n\t"
             "subc.u32 %2, 0, 0;\n\tand.b32 %2, %2, 1;\n\t}"
-            : "=r"(r[K + 0]), "=r"(r[K + 1]), "+r"(c)
+            : "=&r"(r[K + 0]), "=&r"(r[K + 1]), "+r"(c)
             : "r"(a[K + 0]), "r"(a[K + 1]), "r"(b[K + 0]), "r"(b[K + 1]));
     } else {
         asm("{\n\t.reg .u32 t;\n\t"
