@@ -54,10 +54,13 @@ __device__ __forceinline__ void split3(i64 t, i64 N, i64 K, i64 total, i64& n, i
 // (b * R + r) * K + k, or (b * K + k) * R + r when `kmajor` (columns of a GEMM's right operand).
 //
 // Two forms, by the direction of the view's unit stride, so that a warp's loads and stores are runs of consecutive numbers:
-// a warp per row with the lanes along k, or a block of 32 rows (consecutive r) x 8 slices of k.  Either finds the exponent
-// first, then shifts.  (A thread per row walked K numbers one after the other, uncoalesced where k is the unit stride: 480 us
-// for 405 rows of 77 numbers of 42 limbs, 164 for 5,499 columns, now 10 and 41.)
-constexpr int kAlignThreads = 256, kAlignSlices = kAlignThreads / 32;
+// 2^lg lanes per row along k, as many as the row has numbers (a whole warp from K = 17 on), or a block of consecutive rows r x
+// 2^lg slices of k (eight from K = 5 on, one up to 4).  Either finds the exponent first, then shifts.  FULL: the
+// whole warp, the eight slices (constants: 3 us of a product of 9 x 45 x 611 numbers).  (A thread per row walked K
+// numbers one after the other, uncoalesced where k is the unit stride: 480 us for 405 rows of 77 numbers of 42 limbs, 164
+// for 5,499 columns, now 10 and 41.  A warp and eight slices for short rows as well left most of them idle: 200,000 rows
+// of two numbers of 34 limbs 282 us, as columns 71, now 27 and 27; a thread per row 23 and 24.)
+constexpr int kAlignThreads = 256;
 
 template <int L>
 __device__ __forceinline__ void align_one(const int32_t* m, const i64* e, i64 plane, i64 src, i64 E, int32_t* om, i64 oplane, i64 dst) {
@@ -73,53 +76,57 @@ __device__ __forceinline__ void align_one(const int32_t* m, const i64* e, i64 pl
     store_signed<L>(om, oplane, dst, s, neg);
 }
 
-template <int L>
+template <int L, bool FULL>
 __global__ void __launch_bounds__(kAlignThreads) k_align_k(const int32_t* __restrict__ m, const i64* __restrict__ e, i64 plane,
                                                            i64 nbatch, i64 R, i64 K, i64 sb, i64 sr, i64 sk,
                                                            const i64* __restrict__ bidx, int32_t* __restrict__ om,
-                                                           i64* __restrict__ oe, i64 oplane, int kmajor) {
-    const i64 t = (blockIdx.x * (i64)kAlignThreads + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (t >= nbatch * R) return;                                     // whole warps leave together
-    const i64 b = t / R, r = t - b * R, base = (bidx ? bidx[b] : b) * sb + r * sr;
+                                                           i64* __restrict__ oe, i64 oplane, int kmajor, int short_lg) {
+    const int lg = FULL ? 5 : short_lg;
+    const i64 t = (blockIdx.x * (i64)kAlignThreads + threadIdx.x) >> lg;
+    const int lanes = 1 << lg, lane = threadIdx.x & (lanes - 1);
+    const bool in = t < nbatch * R;                                  // the warp stays together for the shuffles
+    const i64 b = in ? t / R : 0, r = in ? t - b * R : 0, base = in ? (bidx ? bidx[b] : b) * sb + r * sr : 0;
     i64 E = EZ;
-    for (i64 k = lane; k < K; k += 32) {
+    for (i64 k = lane; in && k < K; k += lanes) {
         const i64 ek = e[base + k * sk];
         if (ek > E && m[(L - 1) * plane + base + k * sk] != 0) E = ek;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
+        if (o >= lanes) continue;
         const i64 x = __shfl_xor_sync(0xFFFFFFFFu, E, o);
         E = x > E ? x : E;
     }
+    if (!in) return;
     if (lane == 0) oe[t] = E;
-    for (i64 k = lane; k < K; k += 32)
+    for (i64 k = lane; k < K; k += lanes)
         align_one<L>(m, e, plane, base + k * sk, E, om, oplane, kmajor ? (b * K + k) * R + r : t * K + k);
 }
 
-template <int L>
+template <int L, bool FULL>
 __global__ void __launch_bounds__(kAlignThreads) k_align_r(const int32_t* __restrict__ m, const i64* __restrict__ e, i64 plane,
                                                            i64 nbatch, i64 R, i64 K, i64 sb, i64 sr, i64 sk,
                                                            const i64* __restrict__ bidx, int32_t* __restrict__ om,
-                                                           i64* __restrict__ oe, i64 oplane, int kmajor) {
-    __shared__ i64 part[kAlignSlices][32];
-    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
-    const i64 t = blockIdx.x * (i64)32 + lane;
+                                                           i64* __restrict__ oe, i64 oplane, int kmajor, int short_lg) {
+    const int lg = FULL ? 3 : short_lg;
+    __shared__ i64 part[kAlignThreads];                              // [slice][row]
+    const int slices = 1 << lg, nr = kAlignThreads >> lg, x = threadIdx.x & (nr - 1), sl = threadIdx.x >> (8 - lg);
+    const i64 t = blockIdx.x * (i64)nr + x;
     const bool in = t < nbatch * R;
-    const i64 b = in ? t / R : 0, r = t - b * R, base = in ? (bidx ? bidx[b] : b) * sb + r * sr : 0;
+    const i64 b = in ? t / R : 0, r = in ? t - b * R : 0, base = in ? (bidx ? bidx[b] : b) * sb + r * sr : 0;
     i64 E = EZ;
-    if (in)
-        for (i64 k = sl; k < K; k += kAlignSlices) {
-            const i64 ek = e[base + k * sk];
-            if (ek > E && m[(L - 1) * plane + base + k * sk] != 0) E = ek;
-        }
-    part[sl][lane] = E;
-    __syncthreads();
+    for (i64 k = sl; in && k < K; k += slices) {
+        const i64 ek = e[base + k * sk];
+        if (ek > E && m[(L - 1) * plane + base + k * sk] != 0) E = ek;
+    }
+    if (slices > 1) {
+        part[threadIdx.x] = E;
+        __syncthreads();
+        for (int q = 0; q < slices; q++) E = part[q * nr + x] > E ? part[q * nr + x] : E;
+    }
     if (!in) return;
-#pragma unroll
-    for (int x = 0; x < kAlignSlices; x++) E = part[x][lane] > E ? part[x][lane] : E;
     if (sl == 0) oe[t] = E;
-    for (i64 k = sl; k < K; k += kAlignSlices)
+    for (i64 k = sl; k < K; k += slices)
         align_one<L>(m, e, plane, base + k * sk, E, om, oplane, kmajor ? (b * K + k) * R + r : t * K + k);
 }
 
@@ -1105,12 +1112,13 @@ int Launch<L>::align(const int32_t* m, const i64* e, i64 plane, i64 nbatch, i64 
                      const i64* bidx, int32_t* om, i64* oe, i64 oplane, int kmajor, cudaStream_t st) {
     i64 n = nbatch * R;
     if (n == 0) return 0;
-    if (sk == 1 && K > 1) {                              // unit stride along the row
-        k_align_k<L><<<grid_for(n, kAlignThreads / 32), kAlignThreads, 0, st>>>(m, e, plane, nbatch, R, K, sb, sr, sk, bidx, om,
-                                                                               oe, oplane, kmajor);
-    } else {
-        k_align_r<L><<<grid_for(n, 32), kAlignThreads, 0, st>>>(m, e, plane, nbatch, R, K, sb, sr, sk, bidx, om, oe, oplane, kmajor);
-    }
+    const bool along = sk == 1 && K > 1;                 // unit stride along the row
+    int lg = along || K <= 4 ? 0 : 3;
+    while (along && lg < 5 && (1 << lg) < K) lg++;
+    const unsigned grid = grid_for(n, kAlignThreads >> lg);
+    const auto kernel = along ? (lg == 5 ? k_align_k<L, true> : k_align_k<L, false>)
+                              : (lg == 3 ? k_align_r<L, true> : k_align_r<L, false>);
+    kernel<<<grid, kAlignThreads, 0, st>>>(m, e, plane, nbatch, R, K, sb, sr, sk, bidx, om, oe, oplane, kmajor, lg);
     return (int)cudaGetLastError();
 }
 
