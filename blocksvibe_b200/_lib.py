@@ -26,6 +26,7 @@ SIGNATURES = {
     "b3d_moments_stage": [_I, _P, _P, _Q, _P, _P, _Q, _P, _P, _P, _Q, _Q, _Q, _Q, _P, _P, _Q, _P],
     "b3d_moments_flush": [_I, _P, _P, _Q, _P, _Q, _I, _Q, _Q, _I, _P, _P, _I, _I, _I, _I, _P, _P, _Q, _P],
     "b3d_moments_flush_mma": [_I, _P, _P, _Q, _P, _Q, _I, _Q, _Q, _I, _P, _P, _I, _I, _I, _I, _P, _P, _Q, _P, _P],
+    "b3d_moments_flush_form": [_I, _I, _I, _I, _I, _Q, _I, _P],
     "b3d_resize": [_I, _P, _P, _Q, _Q, _I, _P, _P, _Q, _P],
     "b3d_cauchy_align": [_I, _P, _P, _Q, _P, _P, _P, _Q, _P],
     "b3d_cauchy_level2": [_I, _P, _P, _Q, _P, _P, _Q, _P, _P, _P, _Q, _P],

@@ -154,6 +154,14 @@ int b3d_moments_flush_mma(int L, const int32_t* ym, const int64_t* ye, int64_t y
     B3D_DISPATCH_FLUSH(L, cuda_status(MX::flush(a, accumulate, Lout, as_stream(stream)), "b3d_moments_flush_mma"));
 }
 
+int b3d_moments_flush_form(int Lout, int W, int R1, int NN, int KW, int64_t cols, int sms, int* mma) {
+    if (!mma || W < 0 || R1 < 1 || R1 > 32 || NN < 1 || KW < 1 || KW > 12 || !nonneg(cols) || sms < 1)
+        return fail(B3D_E_ARG, "b3d_moments_flush_form: invalid size");
+    b3d::FlushGeom g;
+    *mma = b3d::flush_mma_geom(Lout, W, R1, NN, KW, &g) && b3d::flush_mma_pays(g, Lout, W, R1, KW, cols, sms);
+    return 0;
+}
+
 int b3d_resize(int L, const int32_t* m, const int64_t* e, int64_t plane, int64_t n, int Lout, int32_t* om, int64_t* oe,
                int64_t oplane, void* stream) {
     if (!nonneg(n) || (Lout != L && Lout != L + 4 && Lout != L - 4) || !b3d_supported_limbs(Lout))

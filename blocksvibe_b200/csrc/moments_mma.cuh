@@ -19,9 +19,8 @@
 //
 // What bounds it: latency and integer issue of the limb work around the MMAs (per four columns of R = 11, W = 40: digits
 // 11 K clocks, TMEM to limbs 13 K, sums and rounding 14 K, stores 4 K, the tensor pipe 5 % busy, two CTAs per SM).  The
-// cost of a column grows with R but hardly with W, that of k_moments_flush with W R1, hence the rule of flush(): 1280 bits, R = 27,
-// 170,000 columns: W = 72 12.1 ms against 20.3, W = 32 8.6 against 8.9; 1024 bits, R = 15, W = 48, 300,000 columns 10.6 against
-// 8.3; R = 11, W = 40, 593,400 columns 13.1 against 8.5, 12,500 columns 0.28 against 0.37.
+// cost of a column grows with R but hardly with W, that of k_moments_flush with W R1: which form takes a window is
+// flush_mma_pays, below.
 #pragma once
 #include <atomic>
 #include <cmath>
@@ -421,14 +420,30 @@ __global__ void __launch_bounds__(kFlushMmaThreads, 2) k_moments_flush_mma(Flush
 
 #endif
 
-// Which form, by times of both on a B200 (milliseconds, tensor cores / CUDA cores).  Many columns: the tensor cores from W R1 = 900
-// (1280 bits: W R1 = 896 8.6 / 8.9, 1344 10.7 / 13.4, 768 7.7 / 8.4; 1024 bits: 768 10.6 / 8.3).  Columns that leave the CUDA-core
-// form's thread per column short of threads: 1024 bits, W R1 = 480: 12,500 columns 0.28 / 0.37, 25,000 0.60 / 0.57; 896
-// bits, 224: 8,000 0.13 / 0.21, 20,000 0.28 / 0.24; the line is at 112 columns per SM, from W R1 = 128 (256 bits, 60: 1,800 columns
-// 0.043 / 0.042, 20,000 0.19 / 0.05).
-inline bool flush_mma_pays(int W, int R1, i64 cols) {
+// CTAs resident at a time: two per SM where their shared memory allows (TMEM: 256 of 512 columns each)
+inline i64 flush_mma_slots(const FlushGeom& g, int sms) { return (i64)sms * (g.smem <= 110 * 1024 ? 2 : 1); }
+
+// Which form, by times of both on a B200 (1,344 windows: 6 to 42 limbs, 10 to 100 levels, 2 to 28 orders, 80 to 200,000
+// columns).  The tensor cores need enough levels and terms, and either many terms (a column costs the CUDA cores W R1, the
+// tensor cores R1) or so few columns that the CUDA-core form's thread per column leaves the SMs short of threads.  In
+// microseconds, to 6 and 9 % in the median:
+//     tensor cores  16 + columns per CTA (0.9 + 0.13 R1 + 0.045 LO + 0.00095 W LO)
+//     CUDA cores    20 + W R1 ((0.09 + 0.014 NA) waves + 0.00036 cols NA / 1000)    NA = flush_words, waves >= 1 of the blocks an
+//                                                                                SM's shared memory holds
+// and where the first is well above the second the CUDA cores take the window (milliseconds, tensor / CUDA cores): 256 bits, W = 20,
+// R1 = 7: 12,500 columns 0.15 / 0.08, 500 0.04 / 0.08; 1280 bits, W = 40, R1 = 4, 16,000 columns 0.30 / 0.18; 1280 bits,
+// R1 = 28: 170,000 columns, W = 72 12.1 / 20.3, W = 32 8.6 / 8.9; 1024 bits, R1 = 16, W = 48, 300,000 columns 10.6 / 8.3.
+// The margin of 1.25 keeps every window measured on the tensor cores there whose time the estimates do not settle.
+inline bool flush_mma_pays(const FlushGeom& g, int LO, int W, int R1, int KW, i64 cols, int sms) {
     const i64 terms = (i64)W * R1;
-    return terms >= 900 || (W >= 10 && terms >= 128 && cols < 148 * 112);
+    if (terms < 900 && !(W >= 10 && terms >= 128 && cols < (i64)sms * 112)) return false;
+    const int NA = flush_words(LO, KW);
+    const i64 items = (cols + g.CB - 1) / g.CB, slots = flush_mma_slots(g, sms);
+    const double columns = (double)g.CB * ((items + slots - 1) / slots);
+    const double waves = std::fmax(1.0, (double)cols / (kFlushThreads * (double)sms * (227 / (NA + 1))));
+    const double mma = 16.0 + columns * (0.9 + 0.13 * R1 + 0.045 * LO + 0.00095 * W * LO);
+    const double cuda = 20.0 + (double)terms * ((0.09 + 0.014 * NA) * waves + 0.36e-6 * (double)cols * NA);
+    return mma < 1.25 * cuda;
 }
 
 template <int L>
@@ -438,7 +453,7 @@ struct FlushMmaLaunch {
 
 #ifdef B3D_DEFINE_LAUNCH
 template <int L, int LO>
-static int flush_mma_launch(const FlushMmaArgs& a, const FlushGeom& g, int accumulate, cudaStream_t st) {
+static int flush_mma_launch(const FlushMmaArgs& a, const FlushGeom& g, int sms, int accumulate, cudaStream_t st) {
     static std::atomic<unsigned long long> opted{0};                // devices whose limit is raised
     const unsigned long long dbit = device_bit();
     if (!(opted.load(std::memory_order_relaxed) & dbit) || !dbit) {
@@ -446,12 +461,7 @@ static int flush_mma_launch(const FlushMmaArgs& a, const FlushGeom& g, int accum
         if (rc) return rc;
         opted.fetch_or(dbit, std::memory_order_relaxed);
     }
-    int dev = 0, sms = 0;
-    int rc = (int)cudaGetDevice(&dev);
-    if (!rc) rc = (int)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (rc) return rc;
-    const i64 items = a.rows * ((a.N + g.CB - 1) / g.CB);
-    const i64 slots = (i64)sms * (g.smem <= 110 * 1024 ? 2 : 1);    // TMEM: 256 of 512 columns each
+    const i64 items = a.rows * ((a.N + g.CB - 1) / g.CB), slots = flush_mma_slots(g, sms);
     k_moments_flush_mma<L, LO><<<(unsigned)(items < slots ? items : slots), kFlushMmaThreads, g.smem, st>>>(a, g, accumulate);
     return (int)cudaGetLastError();
 }
@@ -460,9 +470,12 @@ template <int L>
 int FlushMmaLaunch<L>::flush(const FlushMmaArgs& a, int accumulate, int LO, cudaStream_t st) {
     if (a.rows == 0 || a.N == 0 || a.W == 0) return 0;
     FlushGeom g;
-    const bool mma = flush_mma_pays(a.W, a.R1, a.rows * a.N) && flush_mma_geom(LO, a.W, a.R1, a.NN, a.KW, &g);
-    int rc = 0;
-    if (mma) rc = LO == L ? flush_mma_launch<L, L>(a, g, accumulate, st) : flush_mma_launch<L, L + 4>(a, g, accumulate, st);
+    int dev = 0, sms = 0;
+    int rc = (int)cudaGetDevice(&dev);
+    if (!rc) rc = (int)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (rc) return rc;
+    const bool mma = flush_mma_geom(LO, a.W, a.R1, a.NN, a.KW, &g) && flush_mma_pays(g, LO, a.W, a.R1, a.KW, a.rows * a.N, sms);
+    if (mma) rc = LO == L ? flush_mma_launch<L, L>(a, g, sms, accumulate, st) : flush_mma_launch<L, L + 4>(a, g, sms, accumulate, st);
     // all rows, or those with n = 0 in the window (n = m0 + shift there: none once m0 > 0)
     if (!rc && (!mma || a.m0 == 0))
         rc = Launch<L>::moments_flush(a.ym, a.ye, a.yplane, a.row_shift, a.m0, a.W, a.rows, a.N, a.R1, a.nk, a.nkb, a.NN, a.KW,

@@ -136,6 +136,10 @@ int b3d_moments_flush_mma(int L, const int32_t* ym, const int64_t* ye, int64_t y
                           int W, int64_t rows, int64_t N, int R1, const uint32_t* nk, const int32_t* nkb, int NN, int KW,
                           int accumulate, int Lout, int32_t* mm, int64_t* me, int64_t mplane, int* err, void* stream);
 
+/* Which kernel b3d_moments_flush_mma takes for a window of W levels, R1 orders of integers n < NN and cols = rows N columns on a
+ * device of sms multiprocessors: *mma = 1 tensor cores, 0 b3d_moments_flush's.  Host only. */
+int b3d_moments_flush_form(int Lout, int W, int R1, int NN, int KW, int64_t cols, int sms, int* mma);
+
 /* Change of limb count of n numbers, Lout = L or L +- 4: widening is exact, narrowing rounds once (half away from
  * zero).  The derivative stages run with more limbs than the recursion where their sums cancel (the drop-in's
  * choice; no counterpart in the reference, whose stages share one limb count). */
