@@ -897,7 +897,7 @@ __global__ void __launch_bounds__(kMomThreads, 3) k_moments_stage(const int32_t*
 // and exponent.  The grid reaches 32 (LO + 2 + KW) bits below E, the exponent above the chunk's largest term with n^k != 0,
 // and KW + 1 words above it: a term is truncated (towards zero) below 2^(E - 32 (LO + 2)) even after its product with
 // n^k < 2^(32 KW), and |sum| < W 2^(32 KW) 2^E.  A term with n = 0 counts for order 0 only, which then is a chunk
-// of its own.  One rounding per order.
+// of its own.  One rounding per order.  (The kernel's KW is the table's, nkw, rounded up to a compiled one.)
 // Bound by the latency of the carry chains at the eight warps per SM that shared memory leaves room for: the sum of one order
 // and the product for the next run side by side (10.0 ms one after the other; chunks of three orders 8.6, of two 9.4).
 // Before, every word and order had its own offset, bounds check and carry by comparison: 1024 bits, R = 11, W = 40, 593,400 full
@@ -910,7 +910,7 @@ B3D_CX int flush_words(int LO, int KW) { return LO + 2 * KW + 3; }
 template <int L, int LO, int KW, bool ACCUMULATE>
 __global__ void __launch_bounds__(kFlushThreads) k_moments_flush(const int32_t* __restrict__ ym, const i64* __restrict__ ye,
                           i64 yplane, const i64* __restrict__ row_shift, i64 m0, int W, i64 rows, i64 N, int R1,
-                          const u32* __restrict__ nk, const int32_t* __restrict__ nkb, int NN,
+                          const u32* __restrict__ nk, const int32_t* __restrict__ nkb, int NN, int nkw,
                           int32_t* __restrict__ mm, i64* __restrict__ me, i64 mplane, bool zero_rows) {
     constexpr int NB = nb_bits(L);                       // staged terms: L limbs; moments: LO limbs
     constexpr int NA = flush_words(LO, KW), BELOW = 32 * (LO + 2 + KW);
@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(kFlushThreads) k_moments_flush(const int32_t* 
             }
             if (k0 > 0) {                                // u *= n^k0
                 u32 P[NA];
-                const u32* b = nk + ((i64)k0 * NN + n) * KW;
+                const u32* b = nk + ((i64)k0 * NN + n) * nkw;
                 const int nw = (nkb[k0 * NN + n] + 31) >> 5;
                 mul_small(P, u, b[0]);
 #pragma unroll
@@ -1256,7 +1256,7 @@ int Launch<L>::moments_flush(const int32_t* ym, const i64* ye, i64 yplane, const
             opted |= dbit;                                                                                       \
         }                                                                                                    \
         k_moments_flush<L, LOC, KWC, AC><<<grid, kFlushThreads, smem, st>>>(ym, ye, yplane, row_shift, m0, W, rows, N, R1, \
-                                                                            nk, nkb, NN, mm, me, mplane, zero_rows); \
+                                                                            nk, nkb, NN, KW, mm, me, mplane, zero_rows); \
     } while (0)
 #define B3D_FLUSH_KW(LOC) \
     if (KW <= 2) { if (accumulate) B3D_FLUSH(LOC, 2, true); else B3D_FLUSH(LOC, 2, false); } \

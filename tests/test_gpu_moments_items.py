@@ -46,3 +46,25 @@ def test_flush_items_bitwise_equal(cuda, L, dL, W, R1, NN, KW, m0, rows, N, accu
         out.append(mom)
     assert int(err.item()) == 0
     assert torch.equal(out[0].m, out[1].m) and torch.equal(out[0].e, out[1].e)
+
+
+@pytest.mark.parametrize("L,W,R1,NN,KW,wide", [(6, 5, 4, 9, 1, 2), (10, 6, 9, 30, 3, 6), (10, 12, 20, 60, 7, 12), (18, 40, 12, 41, 5, 6)])
+@pytest.mark.parametrize("entry", ["b3d_moments_flush", "b3d_moments_flush_mma"])
+def test_tables_of_any_width(cuda, L, W, R1, NN, KW, wide, entry):
+    """n^k in KW words, not only the widths compiled: the same bits as from a wider table"""
+    rows, N = 9, 4
+    g = torch.Generator().manual_seed(L + W)
+    Y = mpf.random_mpf((W, rows, N), L, spread=30, device=cuda, generator=g)
+    shift = torch.arange(rows, device=cuda) % 3
+    st = torch.cuda.current_stream(cuda).cuda_stream
+    err = torch.zeros(1, dtype=torch.int32, device=cuda)
+    tail = (err.data_ptr(),) if entry.endswith("mma") else ()
+    out = []
+    for kw in (KW, wide):
+        nk, nkb = power_table(R1, NN, kw, cuda)
+        mom = mpf.zeros((rows, R1, N), L, cuda)
+        _lib.call(entry, L, Y.m.data_ptr(), Y.e.data_ptr(), Y.m.stride(0), shift.data_ptr(), 0, W, rows, N, R1, nk.data_ptr(),
+                  nkb.data_ptr(), NN, kw, 0, L, mom.m.data_ptr(), mom.e.data_ptr(), mom.m.stride(0), *tail, st)
+        out.append(mom)
+    assert int(err.item()) == 0
+    assert torch.equal(out[0].m, out[1].m) and torch.equal(out[0].e, out[1].e)
