@@ -22,36 +22,47 @@ from .mpf import MPF
 # default Cauchy kernel and pole-step kernel (see Recursion)
 CAUCHY = "cuda5"
 POLE = "auto"
-# Which pole-step form is faster.  The tensor-core form takes a task's S B columns in chunks of 32 at a cost per
-# chunk that hardly depends on how many columns are in use; the CUDA-core form costs in proportion to the
-# columns.  Measured on a B200 (both forms, both stages, 3000 synthetic tasks per shape, S in {2 .. 5}, S B from 5 to 252):
-# the time ratio CUDA cores / tensor cores of a full chunk, by (L, S); for other column counts the ratio scales with
-# the chunks' fill (S B / (32 chunks)) to within some percent on the low side (half a chunk: 0.96 measured for 0.86).
-POLE_SPEEDUP = {10: (0.67, 0.85, 1.02, 1.11), 18: (0.89, 1.17, 1.44, 1.56), 26: (1.12, 1.45, 1.75, 1.90),
-                30: (1.03, 1.35, 1.57, 1.62), 34: (1.13, 1.45, 1.67, 1.73), 42: (1.25, 1.54, 1.83, 1.37)}   # S = 2, 3, 4, 5
-# The same of the tensor-core kernel that took a row in four warps by turns, pole_mma_gain's model.
+# Which pole-step form is faster.  The tensor-core form takes a task's S B columns in chunks of 32 (one of 16 where there are no
+# more) at a cost per chunk that hardly depends on how many columns are in use; the CUDA-core form costs in
+# proportion to the columns.  Measured on a B200 (both forms, both stages, 1500 to 3000 synthetic tasks per shape, S B of 12 to
+# 64): the time ratio CUDA cores / tensor cores by limb count, of full chunks of 32 columns and of one of 16, S = 2 ... 8.  For
+# other column counts it scales with the chunks' fill, to some percent.  Where S or the limbs grow, fewer CTAs of the
+# tensor-core form fit an SM (34 limbs, S = 6; 42 limbs, S = 8).
+POLE_SPEEDUP = {
+    6: ((0.54, 0.64, 0.73, 0.78, 0.87, 0.97, 1.04), (0.41, 0.49, 0.50, 0.53, 0.64, 0.67, 0.65)),
+    10: ((0.65, 0.78, 0.95, 1.04, 1.12, 1.25, 1.32), (0.50, 0.55, 0.62, 0.66, 0.79, 0.78, 0.81)),
+    14: ((0.72, 0.93, 1.15, 1.25, 1.39, 1.51, 1.63), (0.52, 0.62, 0.70, 0.78, 0.89, 0.91, 0.96)),
+    18: ((0.76, 1.03, 1.23, 1.37, 1.56, 1.67, 1.82), (0.53, 0.66, 0.75, 0.82, 0.98, 0.97, 1.05)),
+    22: ((0.78, 1.05, 1.31, 1.48, 1.66, 1.82, 1.98), (0.54, 0.67, 0.78, 0.88, 1.00, 1.07, 1.16)),
+    26: ((0.89, 1.19, 1.50, 1.68, 1.89, 2.05, 1.72), (0.61, 0.80, 0.90, 1.01, 1.15, 1.20, 1.32)),
+    30: ((0.83, 1.12, 1.35, 1.45, 1.58, 1.25, 1.34), (0.60, 0.73, 0.80, 0.86, 0.95, 0.97, 1.01)),
+    34: ((0.91, 1.22, 1.48, 1.58, 1.30, 1.39, 1.49), (0.61, 0.77, 0.87, 0.95, 1.02, 1.05, 1.12)),
+    38: ((0.90, 1.23, 1.49, 1.15, 1.30, 1.41, 1.51), (0.62, 0.80, 0.90, 0.97, 1.03, 1.08, 0.89)),
+    42: ((0.98, 1.30, 1.61, 1.28, 1.42, 1.55, 0.96), (0.63, 0.81, 0.97, 1.02, 1.11, 0.91, 0.97)),
+    46: ((1.06, 1.32, 1.28, 1.38, 1.50, 0.97, 1.05), (0.67, 0.87, 1.03, 1.06, 1.16, 0.95, 1.03)),
+}
+# The ratios of an earlier tensor-core kernel, S = 2 ... 5, and their model pole_mma_gain: no choice of a run goes by them.
 POLE_FULL_CHUNK_RATIO = {26: (0.71, 0.91, 1.09, 1.23), 30: (0.64, 0.85, 1.02, 1.14), 34: (0.73, 0.93, 1.09, 1.24),
-                         42: (0.90, 1.15, 1.32, 1.51)}            # S = 2, 3, 4, 5
+                         42: (0.90, 1.15, 1.32, 1.51)}
 POLE_MIN_GAIN = 1.05
-
-
-def _chunk_ratio(table, L, S, B):
-    if S < 2:
-        return 0.0
-    Lk = max((k for k in table if k <= L), default=min(table))
-    cols = S * B
-    return table[Lk][min(S, 5) - 2] * cols / (32 * -(-cols // 32))
 
 
 def pole_mma_speedup(L, S, B):
     """predicted time ratio CUDA-core / tensor-core pole step (above 1: the tensor cores are faster)"""
-    return _chunk_ratio(POLE_SPEEDUP, L, S, B)
+    if S < 2:
+        return 0.0
+    full, half = POLE_SPEEDUP[max((k for k in POLE_SPEEDUP if k <= L), default=min(POLE_SPEEDUP))]
+    cols, i = S * B, min(S, 8) - 2
+    return half[i] * cols / 16 if cols <= 16 else full[i] * cols / (32 * -(-cols // 32))
 
 
 def pole_mma_gain(L, S, B):
-    """the ratio by the model of the earlier tensor-core kernel (POLE_FULL_CHUNK_RATIO); the choice of a run goes by
-    pole_mma_speedup"""
-    return _chunk_ratio(POLE_FULL_CHUNK_RATIO, L, S, B)
+    """the ratio of an earlier tensor-core kernel (POLE_FULL_CHUNK_RATIO)"""
+    if S < 2:
+        return 0.0
+    Lk = max((k for k in POLE_FULL_CHUNK_RATIO if k <= L), default=26)
+    cols = S * B
+    return POLE_FULL_CHUNK_RATIO[Lk][min(S, 5) - 2] * cols / (32 * -(-cols // 32))
 
 
 def cauchy_fp_size(L, dmax, nb, Kc, N):
