@@ -144,6 +144,8 @@ class Recursion:
         live = [d for d in self.levels if d]
         self.max_rows = max((d["nb"] * d["Mr"] for d in live), default=0)
         self.max_tasks = max((d["T"] for d in live), default=0)
+        self.max_cols = max((d["nb"] * d["Kc"] for d in live), default=0)        # Cauchy columns of a level
+        self.max_groups = max((d["nb"] for d in live), default=0)
         self._ctable = None
 
     def _cauchy_table(self):
@@ -213,9 +215,15 @@ class Recursion:
                   _lib.ctypes_byref(tabs), p(H.m), p(H.e), H.m.stride(0), stream)
 
     def footprint_bytes(self, B):
-        """device bytes run() allocates for B right-hand sides (slots, Cauchy rows, pole scratch)"""
-        per = (4 * self.L + 8) * self.plan.Smax ** 2 * B
-        return per * (self.plan.nphys + 1 + self.max_rows + self.max_tasks)
+        """device bytes run() allocates for B right-hand sides (slots, Cauchy rows, pole scratch, aligned Cauchy columns)"""
+        N = self.plan.Smax ** 2 * B
+        # one digit buffer for all levels; the other forms allocate per level, a level's buffer before the last one's is freed
+        cols = 8 * self._digits(N) if self.cauchy == "cuda5" else 2 * 4 * self.L * self.max_cols * N
+        return (4 * self.L + 8) * N * (self.plan.nphys + 1 + self.max_rows + self.max_tasks) + cols + 8 * self.max_groups * N
+
+    def _digits(self, N):
+        """doubles of the largest level's digit buffer (the size is proportional to the columns)"""
+        return cauchy_fp_size(self.L, max(self.plan.dmax, 1), 1, self.max_cols, N)
 
     def run(self, h_inf, hook=None, overlap=None):
         """h_inf: MPF (2, >= order, Jh, Smax^2, B).  Returns the residue slots MPF (nphys + 1, Smax^2, B);
@@ -245,6 +253,9 @@ class Recursion:
                 side = self._side[stream] = torch.cuda.Stream(dev)
         pending = None                                   # the side stream's last hook, not yet joined
         use_mma = self.uses_mma(B)
+        if self.cauchy == "cuda5":                       # every level's aligned columns (one stream, one level after the other)
+            Xd = torch.empty(self._digits(N), dtype=torch.float64, device=dev)
+            Xe = torch.empty(max(1, self.max_groups * N), dtype=torch.int64, device=dev)
         p = lambda t: t.data_ptr()
         for lev in self.levels:
             if lev is None:
@@ -255,9 +266,6 @@ class Recursion:
             if self._use_rns(lev):
                 self._cauchy_rns(lev, tabs, res, h_inf, H, stream)
             elif self.cauchy == "cuda5" and lev["m"] > 0:
-                nb, Kc = lev["nb"], lev["Kc"]
-                Xd = torch.empty(cauchy_fp_size(L, plan.dmax, nb, Kc, N), dtype=torch.float64, device=dev)
-                Xe = torch.empty((nb, N), dtype=torch.int64, device=dev)
                 _lib.call("b3d_cauchy_align_fp", L, p(res.m), p(res.e), res.m.stride(0), _lib.ctypes_byref(tabs),
                           plan.dmax, p(Xd), p(Xe), stream)
                 _lib.call("b3d_cauchy_level5", L, p(Xd), p(Xe), p(h_inf.m), p(h_inf.e),
