@@ -537,7 +537,7 @@ def run_ours(args):
     if "b3d_pole_level_mma" in split:
         issued = useful = 0
         for lv in levs:
-            i_, u_ = RL.pole_mma_macs(lv, N, S, L)
+            i_, u_ = RL.pole_mma_issued(lv, N, S, L)
             issued, useful = issued + i_, useful + u_
         reps = 1 if args.schedule == "batched" else len(ns)
         pole_s = split["b3d_pole_level_mma"] / 1e3

@@ -31,8 +31,9 @@ def pole_level_macs(lev, N, S):
 
 
 def pole_mma_geometry(L):
-    """(U, MT): digits per entry along K, padded to whole K steps, and 128-position tiles of the tensor-core pole step
-    (pole_mma.cuh, which packs the entries in chunks of 16 digits: up to 10 % fewer steps than U counts)"""
+    """(U, MT): digits per entry along K where each entry is padded to whole K steps of 32, and 128-position tiles of
+    the tensor-core pole step.  The kernel (pole_mma.cuh) packs entries in chunks of 16 digits: its K steps are
+    pole_mma_steps, up to a quarter fewer (10 limbs, two structures) than U counts."""
     NB, D = 32 * L - 2, 4 * L
     U = 32 * (-(-D // 32))
 
@@ -42,11 +43,25 @@ def pole_mma_geometry(L):
     return U, (1 if 8 * p0(1) + 17 <= NB - 160 else 2)
 
 
-def pole_mma_macs(lev, N, S, L):
+def pole_mma_steps(L, S):
+    """K steps of 32 digits per row of b3d_pole_level_mma: S entries in chunks of 16 digits, two chunks a step"""
+    return (S * (-(-4 * L // 16)) + 1) // 2
+
+
+def pole_mma_issued(lev, N, S, L):
     """int8 MACs of both stages of b3d_pole_level_mma on one level, N = S^2 B numbers per task as in
     pole_level_bytes: (issued by the MMAs, digit products of the exact sums).  A task has S B columns; per task
-    and stage: S rows x S entries x U / 32 K steps x MT tiles of 128 x NC x 32 MACs per column chunk; the exact
-    sums need S^2 (S B) (4 L)^2 digit products."""
+    and stage: S rows x pole_mma_steps x MT tiles of 128 x NC x 32 MACs per column chunk; the exact sums need
+    S^2 (S B) (4 L)^2 digit products."""
+    T = len(lev["t_slot"])
+    cols = N // S
+    nc = 32 if cols >= 32 else 16 * (-(-cols // 16))
+    issued = 2 * T * (-(-cols // nc)) * S * pole_mma_steps(L, S) * pole_mma_geometry(L)[1] * 128 * nc * 32
+    return issued, 2 * T * S * S * cols * (4 * L) ** 2
+
+
+def pole_mma_macs(lev, N, S, L):
+    """pole_mma_issued with each entry padded to whole K steps (pole_mma_geometry's U): more than the kernel issues"""
     U, MT = pole_mma_geometry(L)
     T = len(lev["t_slot"])
     cols = N // S
