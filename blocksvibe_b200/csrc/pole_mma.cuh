@@ -109,9 +109,9 @@ struct PoleMmaSmem {
     }
 };
 
-// v (two's complement, L words) -> balanced base-256 digits, four per word (little-endian bytes, as s8)
 template <int L> B3D_CX bool P0_exact() { return PoleMmaGeom<L>::P0 == 0; }      // nothing is dropped
 
+// v (two's complement, L words) -> balanced base-256 digits, four per word (little-endian bytes, as s8)
 template <int L> __device__ __forceinline__ void to_balanced(u32 (&v)[L]) {
     u32 c = 0;
 #pragma unroll
@@ -134,7 +134,7 @@ __device__ __forceinline__ int pm_jst(const PoleMmaArgs& a) { return a.stage == 
 
 // one column of a row: its positions d4 from P0 -> limbs (two's complement, one more for the sign)
 template <int L>
-__device__ __forceinline__ i64 pm_limbs(const int4* d4, u32 (&w)[PoleMmaGeom<L>::NPW + 1]) {
+B3D_HD i64 pm_limbs(const int4* d4, u32 (&w)[PoleMmaGeom<L>::NPW + 1]) {
     constexpr int NPW = PoleMmaGeom<L>::NPW;
     i64 cy = 0;
 #pragma unroll
@@ -149,24 +149,21 @@ __device__ __forceinline__ i64 pm_limbs(const int4* d4, u32 (&w)[PoleMmaGeom<L>:
     return cy;
 }
 
-// sign, one rounding of a column's limbs, stored at output offset oo
+// sign and one rounding of a column's limbs (value w 2^ein, left as its magnitude): magnitude r, exponent er (EZ: zero).
+// false where a value within the dropped part (2^17 units of w either way) could round differently
 template <int L>
-__device__ __forceinline__ void pm_column(const PoleMmaArgs& a, u32 (&w)[PoleMmaGeom<L>::NPW + 1], i64 E, i64 Er, i64 xo, i64 co,
-                                          i64 oo) {
-    using G = PoleMmaGeom<L>;
-    constexpr int NB = nb_bits(L), NPW = G::NPW, NW = NPW + 1;
+B3D_HD bool pm_round(u32 (&w)[PoleMmaGeom<L>::NPW + 1], i64 ein, u32 (&r)[L], bool* negative, i64* er) {
+    constexpr int NB = nb_bits(L), NPW = PoleMmaGeom<L>::NPW, NW = NPW + 1;
     const bool neg = (w[NPW] >> 31) != 0;
     if (neg) negate(w);
+    *negative = neg;
     // bit length from the top limbs; the half bit of the rounding
     int bl = 0;
 #pragma unroll
     for (int k = NW - 4; k < NW; k++)
-        if (w[k]) bl = 32 * k + 32 - __clz(w[k]);
+        if (w[k]) bl = 32 * k + 32 - clz32(w[k]);
     const int hb = bl - NB - 1, q = hb >> 5, f = hb & 31;
     constexpr int Q0 = (32 * NPW - NB - 1) >> 5;                     // of a sum that fills its limbs; most lie in Q0 - 1, Q0
-    u32 r[L];
-    i64 er;
-    bool done = false;
     if (Q0 >= 3 && bl != 0 && (q == Q0 || q == Q0 - 1)) {
         u32 x[L + 3];                                               // limbs q - 1 .. q + L + 1
 #pragma unroll
@@ -179,34 +176,22 @@ __device__ __forceinline__ void pm_column(const PoleMmaArgs& a, u32 (&w)[PoleMma
 #pragma unroll
         for (int k = 0; k <= L; k++) t[k] = fsr(x[k + 1], x[k + 2], f);
         const u32 half = t[0] & 1u;
-        if (P0_exact<L>() || below != (half ? 0u : ~0u)) {          // no midpoint within the dropped part
+        if (!P0_exact<L>() && below == (half ? 0u : ~0u)) return false;      // a midpoint within the dropped part
 #pragma unroll
-            for (int k = 0; k < L; k++) r[k] = fsr(t[k], t[k + 1], 1);
-            add_bit(r, r, half);
-            int s = hb + 1;
-            if ((r[L - 1] >> (NB - 32 * (L - 1))) != 0) {            // rounded up to 2^NB
+        for (int k = 0; k < L; k++) r[k] = fsr(t[k], t[k + 1], 1);
+        add_bit(r, r, half);
+        int s = hb + 1;
+        if ((r[L - 1] >> (NB - 32 * (L - 1))) != 0) {                // rounded up to 2^NB
 #pragma unroll
-                for (int k = 0; k < L; k++) r[k] = fsr(r[k], k + 1 < L ? r[k + 1] : 0u, 1);
-                s++;
-            }
-            er = E + Er + 8 * G::P0 + s;
-            done = true;
+            for (int k = 0; k < L; k++) r[k] = fsr(r[k], k + 1 < L ? r[k + 1] : 0u, 1);
+            s++;
         }
-    } else if (P0_exact<L>() || round_safe<L, NW, 1>(w)) {           // other lengths: the general rounding
-        if (round_mag<L>(w, E + Er + 8 * G::P0, r, &er)) {
-            done = true;
-        } else {
-            zero(r);
-            er = EZ;
-            done = true;
-        }
+        *er = ein + s;
+        return true;
     }
-    if (!done) {
-        exact_dot<L>(a.cm, a.cplane, co, a.xm, a.xe, a.xplane, xo, pm_jst(a), a.S, E, Er, a.om, a.oe, a.oplane, oo);
-        return;
-    }
-    store_signed<L>(a.om, a.oplane, oo, r, neg && er != EZ);
-    a.oe[oo] = er;
+    if (!P0_exact<L>() && !round_safe<L, NW, 1>(w)) return false;    // other lengths: the general rounding
+    if (!round_mag<L>(w, ein, r, er)) *er = EZ;
+    return true;
 }
 
 // mbarrier wait, bounded, given up early once the CTA has failed
@@ -337,15 +322,23 @@ __global__ void __launch_bounds__(kPoleMmaThreads, 3) k_pole_mma(const __grid_co
                 pm_limbs<L>(reinterpret_cast<const int4*>(dbuf + (lane & (NC - 1)) * DS), wd);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&dempty);
+                // the redo waits for the warp: its call never runs beside lanes that still hold a rounding of their own
+                bool redo = false;
                 if (lane < nn) {
-                    if (E == EZ || Er == EZ) {
-#pragma unroll
-                        for (int k = 0; k < L; k++) a.om[k * a.oplane + oo] = 0;
-                        a.oe[oo] = EZ;
-                    } else {
-                        pm_column<L>(a, wd, E, Er, xbase + co, (crow * S + i) * S, oo);
+                    u32 r[L];
+                    bool neg = false;
+                    i64 er = EZ;
+                    if (E == EZ || Er == EZ) zero(r);
+                    else redo = !pm_round<L>(wd, E + Er + 8 * G::P0, r, &neg, &er);
+                    if (!redo) {
+                        store_signed<L>(a.om, a.oplane, oo, r, neg && er != EZ);
+                        a.oe[oo] = er;
                     }
                 }
+                __syncwarp();
+                if (redo)
+                    exact_dot<L>(a.cm, a.cplane, (crow * S + i) * S, a.xm, a.xe, a.xplane, xbase + co, jst, S, E, Er, a.om, a.oe,
+                                 a.oplane, oo);
             }
         }
     } else {
