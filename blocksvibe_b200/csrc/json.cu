@@ -48,21 +48,7 @@ __global__ void k_emit_text(const char* __restrict__ slots, int stride, const in
 }
 }  // namespace b3d
 
-#define B3D_DISPATCH_DEC(L, CALL)                                              \
-    switch (L) {                                                               \
-        case 6: { using DX = b3d::DecimalLaunch<6>; return CALL; }             \
-        case 10: { using DX = b3d::DecimalLaunch<10>; return CALL; }           \
-        case 18: { using DX = b3d::DecimalLaunch<18>; return CALL; }           \
-        case 26: { using DX = b3d::DecimalLaunch<26>; return CALL; }           \
-        case 30: { using DX = b3d::DecimalLaunch<30>; return CALL; }           \
-        case 34: { using DX = b3d::DecimalLaunch<34>; return CALL; }           \
-        case 14: { using DX = b3d::DecimalLaunch<14>; return CALL; }\
-        case 22: { using DX = b3d::DecimalLaunch<22>; return CALL; }\
-        case 38: { using DX = b3d::DecimalLaunch<38>; return CALL; }\
-        case 46: { using DX = b3d::DecimalLaunch<46>; return CALL; }\
-        case 42: { using DX = b3d::DecimalLaunch<42>; return CALL; }           \
-        default: return b3d::fail(B3D_E_LIMBS, "no kernels compiled for L = " + std::to_string(L)); \
-    }
+#define B3D_DISPATCH_DEC(L, CALL) B3D_DISPATCH_AS(DecimalLaunch, DX, L, CALL)
 
 using b3d::cuda_status;
 using b3d::fail;

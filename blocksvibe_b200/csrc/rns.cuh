@@ -526,8 +526,8 @@ __global__ void __launch_bounds__(256, 2) k_rns_mma4(RnsMma a, RnsTables tb) {
 #endif
 
 // ------------------------------------------------------------------------------------------------
-// 1'. digits on the tensor cores.  One tile = 8 operand rows x 16 columns k (128 elements).  The elements' bytes of the
-// magnitude) form A (128 rows x 4 L bytes, K-major in shared memory); the constant C[(j, t)][d] = byte t of
+// 1'. digits on the tensor cores.  One tile = 8 operand rows x 16 columns k (128 elements).  The magnitude bytes of
+// the elements form A (128 rows x 4 L bytes, K-major in shared memory); the constant C[(j, t)][d] = byte t of
 // (2^(8 d) mod p_j) is B (two tiles of NS rows); S = A B^T holds sum_d byte_d C[(j, t)][d] < 4 L 255^2, so
 // r_j = sum_t S[4 j + t] 2^(8 t) mod p_j (sign applied after).
 //

@@ -262,8 +262,6 @@ int b3d_cauchy_level4(int L, const int32_t* xm, const int64_t* xe, int64_t xplan
                       const int64_t* he, int64_t hplane, const b3d_level_tables* lv, int64_t dmax, int32_t* om,
                       int64_t* oe, int64_t oplane, void* stream);
 
-/* digit matrices of C (as b3d_rns_split writes them) from table[(d + dmax) * np + j] = residues of
- * round(2^(NB-1) / d) */
 /* The Cauchy step in exact double-precision integer arithmetic, the same bits as b3d_cauchy_level4 (replaces
  * cauchy.cauchy, cauchy.py:73-87, like it).  b3d_cauchy_align_fp writes the aligned columns as signed digits (doubles,
  * b3d_cauchy_fp_size of them in the tiled order of csrc/cauchy_fp.cuh, 16-byte aligned) and the column exponents
@@ -275,6 +273,8 @@ int b3d_cauchy_align_fp(int L, const int32_t* rm, const int64_t* re, int64_t rpl
 int b3d_cauchy_level5(int L, const double* xm, const int64_t* xe, const int32_t* hm, const int64_t* he, int64_t hplane,
                       const b3d_level_tables* lv, int64_t dmax, int32_t* om, int64_t* oe, int64_t oplane, void* stream);
 
+/* digit matrices of C (as b3d_rns_split writes them) from table[(d + dmax) * np + j] = residues of
+ * round(2^(NB-1) / d) */
 int b3d_cauchy_digits(const b3d_level_tables* lv, const uint32_t* table, int64_t dmax, int np, int64_t Rp, int64_t Kp,
                       int TR, int64_t mat_bytes, uint8_t* out, void* stream);
 
