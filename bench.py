@@ -153,7 +153,7 @@ class Clocks:
 
 # ---------------------------------------------------------------- kernel probe (launch count, per-kernel events)
 KERNELS_PER_CALL = {"b3d_pole_level": 2, "b3d_pole_level_mma": 2, "b3d_cauchy_align": 2, "b3d_cauchy_align_sm": 2,
-                    "b3d_cauchy_align_fp": 2}
+                    "b3d_cauchy_align_fp": 2, "b3d_cauchy_fp_size": 0, "b3d_moments_flush_form": 0}      # the last two: host only
 
 
 class Probe:
