@@ -325,14 +325,19 @@ __global__ void __launch_bounds__(kPoleMmaThreads, 3) k_pole_mma(const __grid_co
                 // the redo waits for the warp: its call never runs beside lanes that still hold a rounding of their own
                 bool redo = false;
                 if (lane < nn) {
-                    u32 r[L];
-                    bool neg = false;
-                    i64 er = EZ;
-                    if (E == EZ || Er == EZ) zero(r);
-                    else redo = !pm_round<L>(wd, E + Er + 8 * G::P0, r, &neg, &er);
-                    if (!redo) {
-                        store_signed<L>(a.om, a.oplane, oo, r, neg && er != EZ);
-                        a.oe[oo] = er;
+                    if (E == EZ || Er == EZ) {
+#pragma unroll
+                        for (int k = 0; k < L; k++) a.om[k * a.oplane + oo] = 0;
+                        a.oe[oo] = EZ;
+                    } else {
+                        u32 r[L];
+                        bool neg;
+                        i64 er;
+                        redo = !pm_round<L>(wd, E + Er + 8 * G::P0, r, &neg, &er);
+                        if (!redo) {
+                            store_signed<L>(a.om, a.oplane, oo, r, neg && er != EZ);
+                            a.oe[oo] = er;
+                        }
                     }
                 }
                 __syncwarp();
