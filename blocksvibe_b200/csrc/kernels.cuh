@@ -729,15 +729,16 @@ __device__ __forceinline__ void pole_dot(u32* acc, const int32_t* cm, i64 cplane
     for (int k = 0; k < NWF; k++) w[k] = acc[k * kPoleThreads];
     const bool neg = (w[NWF - 1] >> 31) != 0;
     if (neg) negate(w);
-    if (C0 == 0 || round_safe<L, NWF, (C0 > 0 ? 2 : 0)>(w)) {
+    const bool redo = C0 > 0 && !round_safe<L, NWF, (C0 > 0 ? 2 : 0)>(w);
+    if (!redo) {
         u32 r[L];
         i64 er;
         const bool nz = round_mag<L>(w, E + Er + 32 * C0, r, &er);
         store_signed<L>(om, oplane, oo, r, neg && nz);
         oe[oo] = er;
-    } else {
-        exact_dot<L>(cm, cplane, co, xm, xe, xplane, xo, jst, S, E, Er, om, oe, oplane, oo);
     }
+    __syncwarp();                                        // the call runs beside no lane that still has a number to store
+    if (redo) exact_dot<L>(cm, cplane, co, xm, xe, xplane, xo, jst, S, E, Er, om, oe, oplane, oo);
 }
 
 // Pole step, stage 1: Y[t, a, b0, k] = sum_b R[b0, b] H[t_hrow[t], a, b, k]  (R = Rtab[t_R[t]] aligned
