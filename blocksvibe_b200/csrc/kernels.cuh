@@ -649,10 +649,12 @@ __global__ void __launch_bounds__(kCauchyThreads, 4) k_cauchy4(const int32_t* __
 // First try: the product columns from C0 = trunc_cols up, in an accumulator of L + 7 limbs (bits from 32 C0) in shared
 // memory (one column per thread), so that only the operands live in registers.  It lies within 2^(32 (C0 + 2)) of the exact
 // sum; where round_safe shows that no value that close rounds differently, its rounding is the exact sum's.  Elsewhere
-// (heavy cancellation, a sum at a rounding midpoint, exact zeros) exact_dot redoes the sum.  Bound by the integer
-// multiply-add (IMAD.WIDE at half rate: 28 MACs per clock and SM measured) and its latency.  With the 2 L + 2 limbs of
-// the whole sum rounded in registers and the redo unrolled in place the kernels held 168 registers and spilled, three
-// blocks per SM: per 1280-bit task 54.1 ms against 48.8 now, one lambda order at 1024 bits 6.9 against 5.9.
+// (heavy cancellation, a sum at a rounding midpoint, exact zeros) exact_dot redoes the sum.  Bound by the latency of the
+// multiply-add chains and of the operands, which every output loads, negates and shifts anew: 14 limb products per clock
+// and SM over one lambda order at 1024 bits, 18 over a 1280-bit task, of the 32 that the wide multiply at half rate
+// allows (one level at 1024 bits: FMA-heavy pipe half busy, issue 39 %, 17 % of the warps).  With the 2 L + 2 limbs of the
+// whole sum rounded in registers and the redo unrolled in place the kernels held 168 registers and spilled, three blocks
+// per SM: per 1280-bit task 54.1 ms against 48.8 now, one lambda order at 1024 bits 6.9 against 5.9.
 constexpr int kPoleThreads = 128;
 
 template <int L> B3D_CX int pole_win() { return 2 * L + 2 - trunc_cols<L>(); }    // limbs of the first try's accumulator
@@ -901,8 +903,8 @@ __global__ void __launch_bounds__(kMomThreads, 3) k_moments_stage(const int32_t*
 // of its own.  One rounding per order.  (The kernel's KW is the table's, nkw, rounded up to a compiled one.)
 // Bound by the latency of the carry chains at the eight warps per SM that shared memory leaves room for: the sum of one order
 // and the product for the next run side by side (10.0 ms one after the other; chunks of three orders 8.6, of two 9.4).
-// Before, every word and order had its own offset, bounds check and carry by comparison: 1024 bits, R = 11, W = 40, 593,400 full
-// columns 19.7 ms, now 8.1; 1280 bits, R = 27, 170,000 columns: W = 72 43.5 and 20.1, a second window of W = 8 6.4 and 3.7.
+// Before, every word and order had its own offset, bounds check and carry by comparison: 1024 bits, R = 11, W = 40, 593,400
+// columns, every term present 20.8 ms, now 9.0; 1280 bits, R = 27, 170,000 columns: W = 72 43.1 and 18.0, W = 8 5.5 and 2.1.
 constexpr int kFlushThreads = 64;
 constexpr int kFlushKC = 4;
 

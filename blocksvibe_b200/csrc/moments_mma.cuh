@@ -430,9 +430,10 @@ inline i64 flush_mma_slots(const FlushGeom& g, int sms) { return (i64)sms * (g.s
 //     tensor cores  16 + columns per CTA (0.9 + 0.13 R1 + 0.045 LO + 0.00095 W LO)
 //     CUDA cores    20 + W R1 ((0.09 + 0.014 NA) waves + 0.00036 cols NA / 1000)    NA = flush_words, waves >= 1 of the blocks an
 //                                                                                SM's shared memory holds
-// and where the first is well above the second the CUDA cores take the window (milliseconds, tensor / CUDA cores): 256 bits, W = 20,
-// R1 = 7: 12,500 columns 0.15 / 0.08, 500 0.04 / 0.08; 1280 bits, W = 40, R1 = 4, 16,000 columns 0.30 / 0.18; 1280 bits,
-// R1 = 28: 170,000 columns, W = 72 12.1 / 20.3, W = 32 8.6 / 8.9; 1024 bits, R1 = 16, W = 48, 300,000 columns 10.6 / 8.3.
+// and where the first is well above the second the CUDA cores take the window (milliseconds, tensor / CUDA cores, every term
+// present): 256 bits, W = 20, R1 = 7: 12,500 columns 0.15 / 0.08, 500 0.04 / 0.08; 1280 bits, W = 40, R1 = 4, 16,000 columns
+// 0.36 / 0.19; 1280 bits, R1 = 28: 170,000 columns, W = 72 11.8 / 18.0, 200,000 columns, W = 32 9.0 / 10.2; 1024 bits, 200,000
+// columns, R1 = 16, W = 48: 7.0 / 6.4, R1 = 12, W = 40: 4.1 / 3.1.
 // The margin of 1.25 keeps every window measured on the tensor cores there whose time the estimates do not settle.
 inline bool flush_mma_pays(const FlushGeom& g, int LO, int W, int R1, int KW, i64 cols, int sms) {
     const i64 terms = (i64)W * R1;

@@ -28,8 +28,9 @@
 // the slot: the limbs of the sum by one carry chain in registers (the slot is free again), sign, one rounding, coalesced
 // stores, while the front warps multiply the next row.  Slot and rows pass by mbarriers.
 //
-// What bounds it: latency; the MMAs (38 clocks each, their 128-row A operand through shared memory) keep the tensor path
-// busy for a good half of the time at S = 5, L = 34.  Per 1024-bit task (134,316 tasks of 30 columns, both stages): 18.8 ms;
+// What bounds it: latency, one row's windows, MMAs and transposition one after the other; at S = 5, L = 34 the MMAs (38
+// clocks each, their 128-row A operand through shared memory) take 43 % of the time, the tensor pipe counts 20 % of the
+// cycles, issue 30 %.  Per 1024-bit task (134,316 tasks of 30 columns, both stages): 18.4 ms, when first built 18.8;
 // two CTAs of four front and four back warps 22.7 (26.9 and 24.8 with the next item's operands prefetched or preloaded:
 // registers spill), TMEM read 32 columns at a time 26.5 (through local memory).  The form before handled a row in four warps
 // by turns (windows, MMAs, carry segments, one header thread per column, limbs by run-time offsets) with all 256 positions:
