@@ -21,10 +21,10 @@ def flush_form(LO, W, R1, NN, KW, cols, sms=148):
     (30, 20, 7, 81, 2, 12500, 0),                         # 183 / 119
     (46, 40, 4, 81, 2, 16000, 0),                         # 356 / 191
     (46, 72, 28, 81, 6, 16000, 1),                        # 1136 / 2902
-    (46, 72, 28, 81, 6, 170000, 1),                       # 12100 / 20300
+    (46, 72, 28, 81, 6, 170000, 1),                       # 11800 / 18000
     (38, 40, 12, 41, 2, 12500, 1),                        # 280 / 370
-    (38, 40, 12, 41, 2, 593400, 0),                       # 13100 / 8500
-    (38, 48, 16, 49, 6, 300000, 0),                       # 10600 / 8300
+    (38, 40, 12, 41, 2, 593400, 0),                       # 13100 / 9000
+    (38, 48, 16, 49, 6, 300000, 0),                       # 10600 / 8400
     (10, 10, 6, 11, 2, 1800, 0),                          # 43 / 42
     (46, 8, 28, 81, 6, 170000, 0),                        # the second window of an order of 80
     (42, 40, 32, 41, 12, 100, 0),                         # integers too long for one tile
