@@ -178,9 +178,10 @@ _TABLES = {}
 
 def tables(L, device):
     key = (L, str(device))
-    if key not in _TABLES:
-        _TABLES[key] = Tables(L, device)
-    return _TABLES[key]
+    tb = _TABLES.get(key)
+    if tb is None:                       # threads that build at the same time all use the first one stored (its flag is the one read)
+        tb = _TABLES.setdefault(key, Tables(L, device))
+    return tb
 
 
 def _round_up(x, m):

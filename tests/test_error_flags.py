@@ -1,6 +1,7 @@
 """The flags that the tensor-core kernels set when a bounded wait expires (results incomplete) are read wherever results are
 handed over: a flag that the test sets by hand, as an expired wait would, makes each hand-over raise, and stays set
 for the other batches of the operator."""
+import threading
 from types import SimpleNamespace
 
 import pytest
@@ -32,6 +33,26 @@ def test_rns_check_clears_what_it_raises_for(monkeypatch):
     with pytest.raises(_lib.B3DError, match="code 2"):
         rns.check_errors("cpu")
     rns.check_errors(torch.device("cpu"))
+
+
+def test_threads_share_one_table(monkeypatch):
+    """two threads that need a limb count's tables first get the same ones: a flag set in a copy would never be read"""
+    both = threading.Barrier(2)
+
+    class Slow:
+        def __init__(self, L, device):
+            both.wait(10)                                # both are building
+            self.err = flag()
+
+    monkeypatch.setattr(rns, "_TABLES", {})
+    monkeypatch.setattr(rns, "Tables", Slow)
+    got = []
+    ts = [threading.Thread(target=lambda: got.append(rns.tables(6, torch.device("cpu")))) for _ in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert got[0] is got[1] and rns.error_flags("cpu")[0] is got[0].err
 
 
 @pytest.fixture(scope="module")
