@@ -94,10 +94,14 @@ def task_results(tjs, pp, vals, infos, Smax, L, nq):
             for q in range(nq)]
 
 
+class IncompleteResults(_lib.B3DError):
+    """a kernel gave up a bounded wait: the results of its batch are incomplete"""
+
+
 def _raise_codes(codes):
     if any(codes):
-        raise _lib.B3DError(f"a tensor-core kernel did not complete (pole step {codes[0]}, moments flush {codes[1]}, "
-                            f"residue products {codes[2:]})")
+        raise IncompleteResults(f"a tensor-core kernel did not complete (pole step {codes[0]}, moments flush {codes[1]}, "
+                                f"residue products {codes[2:]})")
 
 
 class Operator:
@@ -121,7 +125,7 @@ class Operator:
         return torch.cat([self.rec.err, self.der.err] + rns.error_flags(self.device))
 
     def check_errors(self):
-        """raise B3DError if a kernel of this operator's work gave up a bounded wait: its results are incomplete (waits
+        """raise IncompleteResults if a kernel of this operator's work gave up a bounded wait (waits
         for the current stream).  Every way of handing results to the host does this.  The flags stay set, as batches on
         other streams may share them: the operator is used up; the check_errors of rec, der and the rns module clear."""
         _raise_codes(self._flags().tolist())
@@ -179,7 +183,7 @@ class Operator:
 
     def to_host(self, outs):
         """device results -> host limb arrays through reusable pinned buffers (one D2H copy per array); raises
-        B3DError if a kernel did not complete (check_errors)"""
+        IncompleteResults if a kernel gave up (check_errors)"""
         host = {}
         for c, r in outs.items():
             key = (c, tuple(r.m.shape))
@@ -226,7 +230,7 @@ class GraphStep:
         self.h.e.copy_(self.stage.e.permute(1, 2, 3, 4, 0))
 
     def check_errors(self):
-        """raise B3DError if a kernel of a replay gave up a bounded wait (Operator.check_errors; run() does not wait, so
+        """raise IncompleteResults if a kernel of a replay gave up a bounded wait (Operator.check_errors; run() does not wait, so
         a program that reads `out` itself calls this first)"""
         self.op.check_errors()
 
@@ -259,8 +263,8 @@ class GraphStep:
         batch i's graph runs, so the host transfers overlap the step; the step's stream itself only adds two
         device-to-device copies (inputs into the static buffer, results out of it).  Staging buffers, device
         result copies and host buffers are double-buffered, every reuse ordered by an event; they are allocated on
-        the first call and kept for the next ones.  Raises B3DError in the place of results whose kernels did not
-        complete (Operator.check_errors)."""
+        the first call and kept for the next ones.  Raises IncompleteResults in the place of results whose kernels
+        gave up (Operator.check_errors)."""
         dev = self.op.device
         main = torch.cuda.current_stream(dev)
         if getattr(self, "_pipe", None) is None:               # built once, reused by every call

@@ -208,6 +208,10 @@ class Server:
                         r.result = {(c, d12): x[:, :, :, q:q + 1] for c, x in out.items()}
                     r.done = now
             except Exception as exc:                           # surfaced to the waiting client
+                if isinstance(exc, DI.IncompleteResults):      # its flags stay set: the next request builds the operator anew
+                    with self.lock:
+                        if self.ops.get(key) is op:
+                            del self.ops[key]
                 for r in batch:
                     r.error = exc
                     r.done = time.perf_counter()
